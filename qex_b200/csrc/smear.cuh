@@ -116,27 +116,38 @@ __device__ __forceinline__ bool site_of_thread(const Geom &g, SiteCtx &c) {
   return true;
 }
 
-// S = U_nu(x) F(x+nu) U_nu(x+mu)^dag + U_nu(x-nu)^dag F(x-nu) U_nu(x-nu+mu).
-// Every factor is streamed from memory a row or column at a time, so only
-// the partial product t and S are live 3x3 matrices.
-__device__ __forceinline__ void staple(M3 &S, const Geom &g, const SiteCtx &c, int mu, int nu,
-                                       const double2 *__restrict__ Un, const double2 *__restrict__ F) {
-  const size_t V = (size_t)g.V;
-  const int s_pn = disp1(g, c.x, c.lex, c.par, nu, 1);
-  const int s_pm = disp1(g, c.x, c.lex, c.par, mu, 1);
-  const int s_mn = disp1(g, c.x, c.lex, c.par, nu, -1);
-  const int s_mnpm = disp2(g, c.x, c.lex, c.par, nu, -1, mu, 1);
-  M3 t;
-  // upper: t = U_nu(x) F(x+nu) (column k of U times row k of F); S = t U_nu(x+mu)^dag
+__device__ __forceinline__ void m_zero(M3 &m) {
 #pragma unroll
-  for (int e = 0; e < 9; e++) t.e[e] = make_double2(0.0, 0.0);
+  for (int e = 0; e < 9; e++) m.e[e] = make_double2(0.0, 0.0);
+}
+// r = a b^dag (registers)
+__device__ __forceinline__ void m_nd(M3 &r, const M3 &a, const M3 &b) {
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < 3; k++) s = cjmadd(s, b.e[3 * j + k], a.e[3 * i + k]);
+      r.e[3 * i + j] = s;
+    }
+}
+
+// acc += coef (A B) C^dag of fields A, B, C at sites sa, sb, sc; operands
+// streamed a column / row at a time, so that only the partial product and
+// acc are live 3x3 matrices
+__device__ __forceinline__ void acc_nn_nd(M3 &acc, double coef, const double2 *__restrict__ A, int sa,
+                                          const double2 *__restrict__ B, int sb, const double2 *__restrict__ C,
+                                          int sc, size_t V) {
+  M3 t;
+  m_zero(t);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     double2 a[3], b[3];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      a[j] = __ldg(Un + (size_t)(3 * j + k) * V + c.site);
-      b[j] = __ldg(F + (size_t)(3 * k + j) * V + s_pn);
+      a[j] = __ldg(A + (size_t)(3 * j + k) * V + sa);
+      b[j] = __ldg(B + (size_t)(3 * k + j) * V + sb);
     }
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -145,27 +156,33 @@ __device__ __forceinline__ void staple(M3 &S, const Geom &g, const SiteCtx &c, i
   }
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    double2 cr[3];
+    double2 c[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) cr[k] = __ldg(Un + (size_t)(3 * j + k) * V + s_pm);
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      double2 s = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < 3; k++) s = cjmadd(s, cr[k], t.e[3 * i + k]);  // conj(c_jk) t_ik
-      S.e[3 * i + j] = s;
+    for (int k = 0; k < 3; k++) {
+      c[k] = __ldg(C + (size_t)(3 * j + k) * V + sc);
+      c[k].x *= coef;
+      c[k].y *= coef;
     }
-  }
-  // lower: t = U_nu(x-nu)^dag F(x-nu) (rows k of both); S += t U_nu(x-nu+mu)
 #pragma unroll
-  for (int e = 0; e < 9; e++) t.e[e] = make_double2(0.0, 0.0);
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) acc.e[3 * i + j] = cjmadd(acc.e[3 * i + j], c[k], t.e[3 * i + k]);
+  }
+}
+
+// acc += coef (A^dag B) C
+__device__ __forceinline__ void acc_dn_nn(M3 &acc, double coef, const double2 *__restrict__ A, int sa,
+                                          const double2 *__restrict__ B, int sb, const double2 *__restrict__ C,
+                                          int sc, size_t V) {
+  M3 t;
+  m_zero(t);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     double2 a[3], b[3];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      a[j] = __ldg(Un + (size_t)(3 * k + j) * V + s_mn);
-      b[j] = __ldg(F + (size_t)(3 * k + j) * V + s_mn);
+      a[j] = __ldg(A + (size_t)(3 * k + j) * V + sa);
+      b[j] = __ldg(B + (size_t)(3 * k + j) * V + sb);
     }
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -174,17 +191,38 @@ __device__ __forceinline__ void staple(M3 &S, const Geom &g, const SiteCtx &c, i
   }
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    double2 cr[3];
+    double2 c[3];
 #pragma unroll
-    for (int j = 0; j < 3; j++) cr[j] = __ldg(Un + (size_t)(3 * k + j) * V + s_mnpm);
+    for (int j = 0; j < 3; j++) {
+      c[j] = __ldg(C + (size_t)(3 * k + j) * V + sc);
+      c[j].x *= coef;
+      c[j].y *= coef;
+    }
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-      for (int j = 0; j < 3; j++) S.e[3 * i + j] = cmadd(S.e[3 * i + j], t.e[3 * i + k], cr[j]);
+      for (int j = 0; j < 3; j++) acc.e[3 * i + j] = cmadd(acc.e[3 * i + j], t.e[3 * i + k], c[j]);
   }
 }
 
+// acc += coef St_nu(F), the staple of F along nu for link direction mu:
+// U_nu(x) F(x+nu) U_nu(x+mu)^dag + U_nu(x-nu)^dag F(x-nu) U_nu(x-nu+mu)
+__device__ __forceinline__ void staple_acc(M3 &acc, double coef, const Geom &g, const SiteCtx &c, int mu, int nu,
+                                           const double2 *__restrict__ Un, const double2 *__restrict__ F) {
+  const size_t V = (size_t)g.V;
+  const int s_pn = disp1(g, c.x, c.lex, c.par, nu, 1);
+  const int s_pm = disp1(g, c.x, c.lex, c.par, mu, 1);
+  const int s_mn = disp1(g, c.x, c.lex, c.par, nu, -1);
+  const int s_mnpm = disp2(g, c.x, c.lex, c.par, nu, -1, mu, 1);
+  acc_nn_nd(acc, coef, Un, c.site, F, s_pn, Un, s_pm, V);
+  acc_dn_nn(acc, coef, Un, s_mn, F, s_mn, Un, s_mnpm, V);
+}
+
 __device__ __forceinline__ int other_dir(int mu, int j) { return j < mu ? j : j + 1; }
+// index j of direction d among the three directions other than mu
+__device__ __forceinline__ int other_index(int mu, int d) { return d < mu ? d : d - 1; }
+// field k of an array of link fields
+__device__ __forceinline__ size_t fld(const Geom &g, int k) { return (size_t)k * 9 * g.V; }
 // r-th direction (r = 0, 1) not in {mu, nu}
 __device__ __forceinline__ int third_dir(int mu, int nu, int r) {
   int d = 0, n = 0;
@@ -253,10 +291,19 @@ inline dim3 sweep_grid(const Geom &g) { return dim3((unsigned)(8 * ((g.nh + kSmB
 inline dim3 field_grid(const Geom &g) { return dim3((unsigned)((g.V + kSmBlock - 1) / kSmBlock), 4, 1); }
 
 // makeImpLinks on device fields: u (stride ufs between directions) -> fl
-// (stride ffs); s3 ([4][3][9][V]) and s5 ([4][3][2][9][V]) receive the 3- and
-// 5-staples
+// (stride ffs); s3 and gm ([4][3][9][V] each) receive the 3-staples and the
+// middle fields of the outer staples (null when the level has none)
 int fat7_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, size_t ufs, double2 *fl, size_t ffs,
-             double2 *s3, double2 *s5);
+             double2 *s3, double2 *gm);
+// the level's 3-staples and middle fields alone (a level with five-link terms)
+int fat7_inner_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, size_t ufs, double2 *s3,
+                   double2 *gm);
+// out[mu][j] = St_nu(f_mu), nu = other_dir(mu, j), staples with the links u
+int staples_dev(const Geom &g, const double2 *u, size_t ufs, const double2 *f, size_t fs, double2 *out);
+// out[mu][j] = c0 base_mu + cl f[mu][j] + c5 (f[mu][a] + f[mu][b])
+//              + c7 (St_b(f[mu][a]) + St_a(f[mu][b])), a and b the other two
+int mid_dev(const Geom &g, const double2 *u, size_t ufs, double c0, const double2 *base, size_t bs, double cl,
+            double c5, double c7, const double2 *f, double2 *out);
 int naik_dev(const Geom &g, const double2 *u, size_t ufs, double2 *ll, size_t lfs, double naik);
 int project_u_dev(const Geom &g, const double2 *in, size_t ifs, double2 *out, size_t ofs, double eps);
 
@@ -270,7 +317,7 @@ struct qexstag_smear_s {
 
 namespace qs {
 
-enum SmearSlot { kSmS3 = 0, kSmS5, kSmT1, kSmW, kSmIn0, kSmIn1, kSmOut0, kSmOut1, kSmAos };
+enum SmearSlot { kSmS3 = 0, kSmG, kSmT1, kSmW, kSmIn0, kSmIn1, kSmOut0, kSmOut1, kSmAos };
 
 inline size_t field4_bytes(const Geom &g) { return sizeof(double2) * 9 * (size_t)g.V * 4; }
 
@@ -319,16 +366,19 @@ inline int smear_out_finish(qexstag_smear_s *s, const double2 *dev, double *p, i
   return QEXSTAG_OK;
 }
 
-inline int smear_scratch(qexstag_smear_s *s, const qexstag_fat7_coefs &c, double2 **s3, double2 **s5) {
+// a level with Lepage, 5- or 7-staple terms: the outer staples are of other
+// fields than U itself
+inline bool has_inner(const qexstag_fat7_coefs &c) {
+  return c.five_staple != 0.0 || c.seven_staple != 0.0 || c.lepage != 0.0;
+}
+inline int smear_scratch(qexstag_smear_s *s, const qexstag_fat7_coefs &c, double2 **s3, double2 **gm) {
   const Geom &g = s->l->g;
   const size_t f = sizeof(double2) * 9 * (size_t)g.V;
-  void *p3 = nullptr, *p5 = nullptr;
+  void *p3 = nullptr, *pg = nullptr;
   int rc;
-  const bool have5 = c.five_staple != 0.0 || c.seven_staple != 0.0 || c.lepage != 0.0;
-  if (have5 && (rc = s->ws.get(kSmS3, 12 * f, &p3))) return rc;
-  if (c.seven_staple != 0.0 && (rc = s->ws.get(kSmS5, 24 * f, &p5))) return rc;
+  if (has_inner(c) && ((rc = s->ws.get(kSmS3, 12 * f, &p3)) || (rc = s->ws.get(kSmG, 12 * f, &pg)))) return rc;
   *s3 = (double2 *)p3;
-  *s5 = (double2 *)p5;
+  *gm = (double2 *)pg;
   return QEXSTAG_OK;
 }
 

@@ -8,9 +8,9 @@ library's stream): fat7 with the first-level coefficients (one-link, 3-, 5-,
 7-staple), projectU, fat7 with the second-level coefficients (adds Lepage)
 plus the Naik product, and the whole smear.  Reported per stage: ms,
 algorithmic HBM bytes per site (each link or staple field read and written
-once: sweep 1 reads U and writes 12 3-staple fields and fl, sweep 2 reads U,
-the 3-staples and fl and writes 24 5-staple fields and fl, sweep 3 reads U,
-the 5-staples and fl and writes fl; 144 B per FP64 link) and the achieved
+once: sweep 1 reads U and writes the 12 3-staple fields, sweep 2 reads U and
+those and writes the 12 middle fields of the outer staples, sweep 3 reads U
+and those and writes fl; 144 B per FP64 link) and the achieved
 GB/s, plus QEX's flop count (61632 per site per makeImpLinks,
 src/gauge/fat7l.nim:106) as GF/s.
 """
@@ -27,14 +27,15 @@ from . import stag as S
 
 LINK = 144
 # bytes per site of each stage, all four directions
-FAT7_FULL = 4 * LINK * (1 + 3 + 1) + 4 * LINK * (1 + 3 + 1 + 6 + 1) + 4 * LINK * (1 + 6 + 2)
+FAT7_INNER = 4 * LINK * (1 + 3) + 4 * LINK * (1 + 3 + 3)
+FAT7_FULL = FAT7_INNER + 4 * LINK * (1 + 3 + 1)
 PROJECT = 2 * 4 * LINK
 NAIK = 2 * 4 * LINK
 QEX_FLOPS_FAT7 = 61632
-# adjoint of one fat7 level: sweep A reads M and U, writes 12 T7 fields;
-# sweep B reads M, U, T7, writes 12 M3 fields; sweep C reads M, U, M3, T7,
-# the 12 S3 and 24 S5 forward fields and writes the derivative
-ADJ_FULL = 4 * LINK * (2 + 3) + 4 * LINK * (2 + 3 + 3) + 4 * LINK * (2 + 3 + 3 + 3 + 6 + 1)
+# adjoint of one fat7 level: sweep A reads M and U, writes 12 T fields;
+# sweep B reads U and T, writes 12 M3 fields; sweep C reads M, U, T, M3 and
+# the forward's S and G fields and writes the derivative
+ADJ_FULL = 4 * LINK * (2 + 3) + 4 * LINK * (1 + 3 + 3) + 4 * LINK * (2 + 3 + 3 + 3 + 3 + 1)
 ADJ_NAIK = 4 * LINK  # the long-link chain, read once more by sweep C
 PROJECT_DERIV = 4 * LINK * 4  # reads v, w, the chain; writes the result
 
