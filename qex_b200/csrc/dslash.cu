@@ -14,6 +14,7 @@
 //
 // Compulsory HBM bytes per output site: 8 (naive) or 16 (fat+Naik) links of
 // 144 B, plus 48 B in, 48 B out, plus 48 B per same-site init operand.
+#include <algorithm>
 #include <cstring>
 
 #include "lib.cuh"
@@ -45,6 +46,32 @@ struct DslashArgs64 {
   int rowlen, pitch;
 };
 
+// j-th output site of the launch, as an index of the parity block
+__device__ __forceinline__ int out_site(const DslashArgs64 &A, int j) {
+  if (A.rowlen > 0) {
+    const int q = j / A.rowlen;
+    return A.k0 + q * A.pitch + (j - q * A.rowlen);
+  }
+  return j < A.n1 ? A.k0 + j : A.k2 + (j - A.n1);
+}
+
+// the sum over the grid of each thread's part of <p, Ap>
+template <int RED>
+__device__ __forceinline__ void reduce_pap(const DslashArgs64 &A, double dot) {
+  double v[1] = {dot}, s[1];
+  if (grid_reduce<1>(v, A.partials, A.ticket, s) && threadIdx.x == 0) {
+    if (RED == kRedCgPAp) {
+      // cg.nim:213-215: qLAp = <q, LAp>, alpha = rz/qLAp; itn counted at Ap
+      CgState *st = A.state;
+      st->pAp = s[0];
+      st->alpha = st->rz / s[0];
+      st->itn += 1;
+    } else {
+      *A.dot_out = s[0];
+    }
+  }
+}
+
 template <int NL, int HOP, int INIT, int RED>
 __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) {
   pdl_wait();
@@ -56,13 +83,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
   const size_t out_base = (size_t)A.po * nh;
   double dot = 0.0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < A.nsites; j += gridDim.x * blockDim.x) {
-    int k;
-    if (A.rowlen > 0) {
-      const int q = j / A.rowlen;
-      k = A.k0 + q * A.pitch + (j - q * A.rowlen);
-    } else {
-      k = j < A.n1 ? A.k0 + j : A.k2 + (j - A.n1);
-    }
+    const int k = out_site(A, j);
     int x[4], lex;
     site_coords(g, A.po, k, x, lex);
     double2 acc[3];
@@ -137,34 +158,135 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
       }
     }
   }
-  if (RED != kRedNone) {
-    double v[1] = {dot}, s[1];
-    if (grid_reduce<1>(v, A.partials, A.ticket, s) && threadIdx.x == 0) {
-      if (RED == kRedCgPAp) {
-        // cg.nim:213-215: qLAp = <q, LAp>, alpha = rz/qLAp; itn counted at Ap
-        CgState *st = A.state;
-        st->pAp = s[0];
-        st->alpha = st->rz / s[0];
-        st->itn += 1;
-      } else {
-        *A.dot_out = s[0];
-      }
-    }
-  }
-  (void)out_base;
+  if (RED != kRedNone) reduce_pap<RED>(A, dot);
 }
 
+// The same half sweep with a site's hops spread over the eight warps of a
+// block: 32 sites per block step, warp w forming one link's two products
+// (fat+Naik) or one of them (naive) for all 32, through shared memory to the
+// threads (colour, site) that add them.  The products and the order of their
+// sum are those of dslash64_kernel, so the result is the same bit for bit.
+//
+// Where the whole-site kernel has too few blocks to fill the GPU, its time
+// is one thread's walk through 8 or 16 dependent rounds of loads; this form
+// takes one or two rounds.  Schur operator (two sweeps), us, whole-site form
+// against this one: 8^4 naive 13.3 / 8.3, 8^3 x 16 fat+Naik 45.5 / 9.6, 16^4
+// fat+Naik 64.6 / 35.2.  With the GPU full it loses to the meeting in shared
+// memory (32^4 fat+Naik 426 / 446).
+constexpr int kSplitSites = 32;
+constexpr int kSplitWarps = kBlock / 32;
+
 template <int NL, int HOP, int INIT, int RED>
-static void launch64(const DslashArgs64 &A, int grid) {
-  launch_pdl(dslash64_kernel<NL, HOP, INIT, RED>, grid, kBlock, A);
+__global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs64 A) {
+  constexpr int kTerms = 2 * NL, kPer = kTerms / kSplitWarps;
+  __shared__ double2 term[kTerms][3][kSplitSites];
+  pdl_wait();
+  if (A.done != nullptr && *A.done) return;
+  const Geom &g = A.g;
+  const int nh = g.nh;
+  const size_t V = (size_t)g.V;
+  const size_t in_base = (size_t)(1 - A.po) * nh;
+  const size_t out_base = (size_t)A.po * nh;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double dot = 0.0;
+  for (int j0 = blockIdx.x * kSplitSites; j0 < A.nsites; j0 += gridDim.x * kSplitSites) {
+    const bool on = j0 + lane < A.nsites;
+    const int k = out_site(A, on ? j0 + lane : j0);
+    int x[4], lex;
+    site_coords(g, A.po, k, x, lex);
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+      const int n = w * kPer + q, l = n >> 1;  // term n: link l, forward (even n) or backward
+      const int mu = NL == 8 ? (l >> 1) : l, len = (NL == 8 && (l & 1)) ? 3 : 1;
+      const double2 *ul = A.u + (size_t)l * 9 * V;
+      double2 v[3], m[9], t[3];
+      if ((n & 1) == 0) {
+        const int jf = (lex + lex_step(g, x, mu, len)) >> 1;
+#pragma unroll
+        for (int e = 0; e < 9; e++) m[e] = ldlink(ul + (size_t)e * V + out_base + k);
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + jf);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          t[i] = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int c = 0; c < 3; c++) t[i] = cmadd(t[i], m[3 * i + c], v[c]);
+        }
+      } else {
+        const int jb = (lex + lex_step(g, x, mu, -len)) >> 1;
+#pragma unroll
+        for (int e = 0; e < 9; e++) m[e] = ldlink(ul + (size_t)e * V + in_base + jb);
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + jb);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          t[i] = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int c = 0; c < 3; c++) t[i] = cjmadd(t[i], m[3 * c + i], v[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) term[n][c][lane] = t[c];
+    }
+    __syncthreads();
+    if (w < 3 && on) {
+      const int c = w;
+      double2 acc = make_double2(0.0, 0.0), xsv = acc;
+      if (INIT > 0) {
+        xsv = __ldcg(A.xs + (size_t)c * A.sstride + k);
+        acc = make_double2(A.b * xsv.x, A.b * xsv.y);
+      }
+      if (INIT == 2) {
+        const double2 rv = __ldcg(A.rin + (size_t)c * A.rstride + k);
+        acc.x = fma(A.a, rv.x, acc.x);
+        acc.y = fma(A.a, rv.y, acc.y);
+      }
+#pragma unroll
+      for (int n = 0; n < kTerms; n++) {
+        const double2 t = term[n][c][lane];
+        if ((HOP > 0) == ((n & 1) == 0)) {
+          acc.x += t.x;
+          acc.y += t.y;
+        } else {
+          acc.x -= t.x;
+          acc.y -= t.y;
+        }
+      }
+      const double2 o = make_double2(A.c * acc.x, A.c * acc.y);
+      A.out[(size_t)c * A.ostride + k] = o;
+      if (RED != kRedNone) {
+        dot = fma(xsv.x, o.x, dot);
+        dot = fma(xsv.y, o.y, dot);
+      }
+    }
+    __syncthreads();
+  }
+  if (RED != kRedNone) reduce_pap<RED>(A, dot);
+}
+
+// Sites per launch up to which a half sweep spreads each site over a block's
+// warps: between the last lattice measured faster that way and the first
+// measured slower (Schur us, whole-site / split; fat+Naik: 24^4 145.6 / 137.9,
+// 24^3 x 32 165.5 / 185.1; naive: 16^3 x 32 39.4 / 35.6, 20^4 41.5 / 42.3).
+template <int NL>
+constexpr int kSplitMax = NL == 8 ? 196608 : 65536;
+
+template <int NL, int HOP, int INIT, int RED>
+static void launch64(const DslashArgs64 &A) {
+  if (A.nsites <= kSplitMax<NL>) {
+    const int grid = std::min((A.nsites + kSplitSites - 1) / kSplitSites, num_sms() * 3);
+    launch_pdl(dslash64_split_kernel<NL, HOP, INIT, RED>, grid, kBlock, A);
+  } else {
+    launch_pdl(dslash64_kernel<NL, HOP, INIT, RED>, grid_for(A.nsites, kBlock, 6), kBlock, A);
+  }
   note_launch();
 }
 
 template <int NL>
-static int dispatch64(const DslashArgs64 &A, int hop, int init, int red, int grid) {
+static int dispatch64(const DslashArgs64 &A, int hop, int init, int red) {
 #define QS_D64(H, I, R)                                            \
   if (hop == H && init == I && red == R) {                         \
-    launch64<NL, H, I, R>(A, grid);                                \
+    launch64<NL, H, I, R>(A);                                \
     return QEXSTAG_OK;                                             \
   }
   QS_D64(1, 0, kRedNone)
@@ -206,10 +328,7 @@ int dslash64(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, C
   A.k0 = A.k2 = 0;
   A.n1 = A.nsites = g.nh;
   A.rowlen = A.pitch = 0;
-  int grid = grid_for(g.nh, kBlock, 6);
-  if (red != kRedNone && grid > kMaxRedBlocks) grid = kMaxRedBlocks;
-  int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, red, grid)
-                         : dispatch64<4>(A, hop, init, red, grid);
+  int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, red) : dispatch64<4>(A, hop, init, red);
   if (rc) return rc;
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
@@ -245,8 +364,7 @@ int dslash64_ranges(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVec
   A.nsites = (k1 - k0) + (k3 - k2);
   if (A.nsites == 0) return QEXSTAG_OK;
   const int init = xs.p ? 1 : 0;
-  const int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, kRedNone, grid_for(A.nsites, kBlock, 6))
-                               : dispatch64<4>(A, hop, init, kRedNone, grid_for(A.nsites, kBlock, 6));
+  const int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, kRedNone) : dispatch64<4>(A, hop, init, kRedNone);
   if (rc) return rc;
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
@@ -282,8 +400,7 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
   A.n1 = A.nsites;
   if (A.nsites == 0) return QEXSTAG_OK;
   const int init = xs.p ? 1 : 0;
-  const int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, kRedNone, grid_for(A.nsites, kBlock, 6))
-                               : dispatch64<4>(A, hop, init, kRedNone, grid_for(A.nsites, kBlock, 6));
+  const int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, kRedNone) : dispatch64<4>(A, hop, init, kRedNone);
   if (rc) return rc;
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
@@ -314,7 +431,6 @@ int schur64_plain(const qexstag_links_s *gl, int par, VecD r, CVecD x, VecD t, d
   A.g = g;
   A.u = gl->u64;
   A.n1 = A.nsites = g.nh;
-  const int grid = grid_for(g.nh, kBlock, 6);
   // t = (2D)_{q,par} x
   A.po = 1 - par;
   A.xin = x.p;
@@ -323,9 +439,9 @@ int schur64_plain(const qexstag_links_s *gl, int par, VecD r, CVecD x, VecD t, d
   A.ostride = t.stride;
   A.c = 1.0;
   if (gl->nl == 8)
-    launch64<8, 1, 0, kRedNone>(A, grid);
+    launch64<8, 1, 0, kRedNone>(A);
   else
-    launch64<4, 1, 0, kRedNone>(A, grid);
+    launch64<4, 1, 0, kRedNone>(A);
   // r = 4 m2 x - (2D)_{par,q} t
   A.po = par;
   A.xin = t.p;
@@ -336,9 +452,9 @@ int schur64_plain(const qexstag_links_s *gl, int par, VecD r, CVecD x, VecD t, d
   A.ostride = r.stride;
   A.b = 4.0 * m2;
   if (gl->nl == 8)
-    launch64<8, -1, 1, kRedNone>(A, grid);
+    launch64<8, -1, 1, kRedNone>(A);
   else
-    launch64<4, -1, 1, kRedNone>(A, grid);
+    launch64<4, -1, 1, kRedNone>(A);
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
 }

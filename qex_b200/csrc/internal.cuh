@@ -83,6 +83,20 @@ __device__ __forceinline__ int nbr_half(const Geom &g, const int x[4], int lex, 
   return (lex + (xn - xm) * g.stride[mu]) >> 1;
 }
 
+// (selects instead of indexing x[] with a runtime direction, which would put
+// the coordinates in local memory)
+__device__ __forceinline__ int pick(const int v[4], int d) {
+  return d == 0 ? v[0] : d == 1 ? v[1] : d == 2 ? v[2] : v[3];
+}
+// lex offset of moving a steps along mu from coordinate xm (periodic)
+__device__ __forceinline__ int lex_step(const Geom &g, const int x[4], int mu, int a) {
+  const int xm = pick(x, mu), Lm = pick(g.L, mu);
+  int y = xm + a;
+  if (y >= Lm) y -= Lm;
+  if (y < 0) y += Lm;
+  return (y - xm) * pick(g.stride, mu);
+}
+
 template <int NL>
 struct Hop {
   static __device__ __forceinline__ int mu(int l) { return NL == 8 ? (l >> 1) : l; }

@@ -72,19 +72,6 @@ __device__ __forceinline__ void m_dn(M3 &r, const M3 &a, const M3 &b) {
 
 // Site index of x + a*mu (periodic): lex moves by the wrapped step, the
 // parity flips with a odd (all L even).
-// (selects instead of indexing x[] with a runtime direction, which would put
-// the coordinates in local memory)
-__device__ __forceinline__ int pick(const int v[4], int d) {
-  return d == 0 ? v[0] : d == 1 ? v[1] : d == 2 ? v[2] : v[3];
-}
-// lex offset of moving a steps along mu from coordinate xm (periodic)
-__device__ __forceinline__ int lex_step(const Geom &g, const int x[4], int mu, int a) {
-  const int xm = pick(x, mu), Lm = pick(g.L, mu);
-  int y = xm + a;
-  if (y >= Lm) y -= Lm;
-  if (y < 0) y += Lm;
-  return (y - xm) * pick(g.stride, mu);
-}
 __device__ __forceinline__ int disp1(const Geom &g, const int x[4], int lex, int par, int mu, int a) {
   const int l = lex + lex_step(g, x, mu, a);
   return (l >> 1) + (((par ^ a) & 1) ? g.nh : 0);

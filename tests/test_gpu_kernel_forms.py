@@ -1,0 +1,35 @@
+"""The forms a kernel takes by size, at the sizes where one can go wrong: tile
+remainders, the smallest and largest lattice of each form.  FP64 kernels with
+another order of accumulation than the oracle's: 1e-13 of the largest entry."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from qex_b200 import fields as F
+from qex_b200 import stag as S
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return np.abs(a - b).max() / np.abs(b).max()
+
+
+# half sweeps: 4^4 (128 sites a parity), 720 = 22 1/2 sets of 32 sites, 65536
+# (the last naive lattice spread over warps) and 69632 (the first that is not)
+@pytest.mark.parametrize("dims,naik", [((4, 4, 4, 4), 0), ((4, 6, 6, 10), 0), ((4, 6, 6, 10), 1),
+                                       ((16, 16, 16, 32), 0), ((16, 16, 16, 34), 0)])
+def test_half_sweep_forms(cuda, dims, naik):
+    g = F.fat_naik_links(dims, 3) if naik else F.naive_links(dims, 0.3, 3)
+    V = F.volume(dims)
+    o, s = O.Oracle(dims, g), S.Staggered(S.Layout(dims), S.to_device_links(g))
+    x, r0 = F.gaussian_vector(V, 4), F.gaussian_vector(V, 5)
+    for par in (0, 1):
+        r, ro = S.to_device_vector(r0), r0.copy()
+        s.stagD2(par, r, S.to_device_vector(x), 0.3, 0.7)
+        o.stagD2(par, ro, x, 0.3, 0.7)
+        assert rel(S.to_host_vector(r), ro) < 1e-13
+    r, ro = S.to_device_vector(np.zeros_like(x)), o.vec()
+    s.stagD2ee(r, S.to_device_vector(x), 0.01)
+    o.stagD2ee(ro, x, 0.01)
+    assert rel(S.to_host_vector(r), ro) < 1e-13
