@@ -6,13 +6,13 @@
 // (src/maths/matrixFunctions.nim:368-390) and fat7lDeriv again.
 //
 // Here each fat7 level, in the form of smear.cu (S_nu = St_nu(U_mu), G_nu,
-// fl = c1' U + sum_nu St_nu(G_nu)), is differentiated in three gather sweeps
-// over (site, direction), with S and G from the forward sweeps.  With M the
+// fl = c1' U + sum_nu St_nu(G_nu)), is differentiated in four sweeps over
+// (site, direction), with S and G from the forward sweeps.  With M the
 // chain on the fat links:
 //   T_nu  = St_nu(M_mu)                                (chain on G_nu)
 //   M3_nu = cL T_nu + c5 (T_a + T_b) + c7 (St_b(T_a) + St_a(T_b))
 //                                                      (chain on S_nu)
-// are the forward's own first two sweeps run on M, and the last sweep is
+// are the forward's own first two sweeps run on M, and the last two form
 //   dU_d(y) = c1' M_d + sum_nu (c3 T_nu + St_nu(M3_nu))   (U_d the middle link)
 //             + the derivatives of the staples in which U_d is a side link,
 //               for each other direction mu: the outer staple along d (chain
@@ -20,9 +20,6 @@
 //               S_b, and a, b exchanged) and the 3-staple (chain M3_d,
 //               middle U_mu)
 //             + the Naik product's three positions.
-// Every field is stored once and read as it is; with sums of up to five
-// fields formed at each read, and the 5-staples among them, the whole chain
-// rule took 3.34 ms on 12 x 20 x 14 x 18, now 2.07 ms.
 // St(g; F) = g(x) F(x+nu) g(x+mu)^dag + g(x-nu)^dag F(x-nu) g(x-nu+mu) is the
 // staple of the field F along nu; it is also its own adjoint in F, which is
 // why the chains on the inner staples are staples of the outer chains.  The
@@ -30,25 +27,17 @@
 // with respect to the side field at y is
 //   c(y) g1(y+d2) g2(y+d1)^dag + g2(y) g1(y+d2) c(y+d1)^dag
 //   + c(y-d2)^dag g1(y-d2) g2(y-d2+d1) + g2(y-d2)^dag g1(y-d2) c(y-d2+d1),
-// so every derivative is gathered at its own site: no atomics, no scatter.
+// that is, with z = y-d2, two terms of y's own operands at y and y+d1 and two
+// of z's at z and z+d1.  Gathered at y they read every field at four sites.
+// Here a thread forms, from its operands at y and y+d1, the two terms of y
+// and the two that belong to y+d2; the latter go to a field of their own
+// (one per pair of directions) that the last sweep reads: no atomics, and
+// half the matrices through L2, which bounds these sweeps.  Chain rule on
+// 12 x 20 x 14 x 18: 3.33 ms with up to five fields summed at each gather,
+// 2.07 with single fields, 1.87 with the terms formed at their operands.
 #include "smear.cuh"
 
 namespace qs {
-
-// acc += coef d/dg1 [chain C on St(g1; G2)] at y, g1 the side field of this
-// thread's direction d (= d1), G2 of link direction d2
-__device__ __forceinline__ void side_acc(M3 &acc, double coef, const Geom &g, const SiteCtx &c, int d, int d2,
-                                         const double2 *g1, const double2 *G2, const double2 *C) {
-  const size_t V = (size_t)g.V;
-  const int s_p2 = disp1(g, c.x, c.lex, c.par, d2, 1);
-  const int s_p1 = disp1(g, c.x, c.lex, c.par, d, 1);
-  const int s_m2 = disp1(g, c.x, c.lex, c.par, d2, -1);
-  const int s_m2p1 = disp2(g, c.x, c.lex, c.par, d2, -1, d, 1);
-  acc_nn_nd(acc, coef, C, c.site, g1, s_p2, G2, s_p1, V);
-  acc_nn_nd(acc, coef, G2, c.site, g1, s_p2, C, s_p1, V);
-  acc_dn_nn(acc, coef, C, s_m2, g1, s_m2, G2, s_m2p1, V);
-  acc_dn_nn(acc, coef, G2, s_m2, g1, s_m2, C, s_m2p1, V);
-}
 
 struct AdjArgs {
   Geom g;
@@ -67,10 +56,118 @@ struct AdjArgs {
   size_t dfs;
   int accumulate;     // add to d instead of overwriting it
   double c1, c3, c7;
-  int inner;
+  int inner, side;
+  double2 *q;         // [4][3][9][V] side terms on their way to y + mu
 };
 
-// the derivative with respect to U_d at y
+// One product of the side derivatives with chain or middle fields A at y and
+// B at y + d, g1 the side field's links:
+//   p += coef A(y) g1(y+mu) B(y+d)^dag        (belongs to y)
+//   q += coef A(y)^dag g1(y) B(y+d)           (belongs to y + mu)
+__device__ __forceinline__ void side_term(M3 &p, M3 &q, double coef, const double2 *__restrict__ A, int sy,
+                                          const double2 *__restrict__ B, int syd, const double2 *__restrict__ g1,
+                                          int symu, size_t V) {
+  M3 b, t;
+  m_load(b, B, V, syd);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    double2 r[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      r[k] = __ldg(g1 + (size_t)(3 * i + k) * V + symu);
+      r[k].x *= coef;
+      r[k].y *= coef;
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < 3; k++) s = cjmadd(s, b.e[3 * j + k], r[k]);
+      t.e[3 * i + j] = s;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double2 a[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) a[i] = __ldg(A + (size_t)(3 * i + k) * V + sy);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) p.e[3 * i + j] = cmadd(p.e[3 * i + j], a[i], t.e[3 * k + j]);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double2 r[3], u[3];
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+      r[l] = __ldg(g1 + (size_t)(3 * k + l) * V + sy);
+      r[l].x *= coef;
+      r[l].y *= coef;
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      u[j] = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int l = 0; l < 3; l++) u[j] = cmadd(u[j], r[l], b.e[3 * l + j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double2 a = __ldg(A + (size_t)(3 * k + i) * V + sy);
+#pragma unroll
+      for (int j = 0; j < 3; j++) q.e[3 * i + j] = cjmadd(q.e[3 * i + j], a, u[j]);
+    }
+  }
+}
+
+// the side terms with U_d: those of y go to d_d(y), those of y + mu to
+// q[d][mu](y), which the last sweep picks up.  255 registers and 8 warps an
+// SM: 306 us on 12 x 20 x 14 x 18, against 371 us at 168 registers and 12
+// warps, which spill.
+__global__ void __launch_bounds__(kSmBlock, 2) fat7_adj_side_kernel(const AdjArgs A) {
+  SiteCtx c;
+  if (!site_of_thread(A.g, c)) return;
+  const int d = c.mu;
+  const Geom &g = A.g;
+  const size_t V = (size_t)g.V;
+  const double2 *Ud = A.u + d * A.ufs;
+  M3 p;
+  m_zero(p);
+  if (A.accumulate) m_load(p, A.d + d * A.dfs, V, c.site);
+  const int syd = disp1(g, c.x, c.lex, c.par, d, 1);
+#pragma unroll 1
+  for (int jm = 0; jm < 3; jm++) {
+    const int mu = other_dir(d, jm);
+    const int symu = disp1(g, c.x, c.lex, c.par, mu, 1);
+    const int ja = mu * 3 + other_index(mu, third_dir(mu, d, 0)), jb = mu * 3 + other_index(mu, third_dir(mu, d, 1));
+    const int jd = mu * 3 + other_index(mu, d);
+    M3 q;
+    m_zero(q);
+    const int np = !A.inner ? 1 : A.c7 != 0.0 ? 4 : 2;
+#pragma unroll 1
+    for (int k = 0; k < 2 * np; k++) {
+      // pair k / 2 of chain and middle field, as (chain, middle) and (middle, chain)
+      const double2 *C = A.m + mu * A.mfs, *G = A.u + mu * A.ufs;
+      double coef = A.c3;
+      if (A.inner) {
+        const int pr = k >> 1;
+        coef = pr < 2 ? 1.0 : A.c7;
+        if (pr == 0) G = A.gm + fld(g, jd);
+        if (pr == 1) C = A.m3 + fld(g, jd);
+        if (pr >= 2) {
+          C = A.t7 + fld(g, pr == 2 ? ja : jb);
+          G = A.s3 + fld(g, pr == 2 ? jb : ja);
+        }
+      }
+      side_term(p, q, coef, (k & 1) ? G : C, c.site, (k & 1) ? C : G, syd, Ud, symu, V);
+    }
+    m_store(A.q + fld(g, d * 3 + jm), V, c.site, q);
+  }
+  m_store(A.d + d * A.dfs, V, c.site, p);
+}
+
+// the derivative with respect to U_d at y: the side terms, U_d as the middle
+// link, and the Naik product
 __global__ void __launch_bounds__(kSmBlock, 3) fat7_adj_link_kernel(const AdjArgs A) {
   SiteCtx c;
   if (!site_of_thread(A.g, c)) return;
@@ -80,42 +177,28 @@ __global__ void __launch_bounds__(kSmBlock, 3) fat7_adj_link_kernel(const AdjArg
   const double2 *Ud = A.u + d * A.ufs;
   M3 acc;
   m_zero(acc);
-  if (A.accumulate) m_load(acc, A.d + d * A.dfs, V, c.site);
+  if (A.accumulate || A.side) {
+#pragma unroll
+    for (int e = 0; e < 9; e++) acc.e[e] = A.d[d * A.dfs + (size_t)e * V + c.site];
+  }
   {
     M3 md;
     m_load(md, A.m + d * A.mfs, V, c.site);
     m_axpy(acc, A.c1, md);
   }
-  if (A.inner) {
+  if (A.side) {
 #pragma unroll 1
     for (int j = 0; j < 3; j++) {
       const int nu = other_dir(d, j);
-      if (A.c3 != 0.0) {
-        M3 t;
+      M3 t;
+      m_load(t, A.q + fld(g, d * 3 + j), V, disp1(g, c.x, c.lex, c.par, nu, -1));
+      m_axpy(acc, 1.0, t);
+      if (A.inner && A.c3 != 0.0) {
         m_load(t, A.t7 + fld(g, d * 3 + j), V, c.site);
         m_axpy(acc, A.c3, t);
       }
-      staple_acc(acc, 1.0, g, c, d, nu, A.u + nu * A.ufs, A.m3 + fld(g, d * 3 + j));
-    }
-#pragma unroll 1
-    for (int jm = 0; jm < 3; jm++) {
-      const int mu = other_dir(d, jm);
-      const int jd = mu * 3 + other_index(mu, d);
-      side_acc(acc, 1.0, g, c, d, mu, Ud, A.u + mu * A.ufs, A.m3 + fld(g, jd));
-      side_acc(acc, 1.0, g, c, d, mu, Ud, A.gm + fld(g, jd), A.m + mu * A.mfs);
-      if (A.c7 != 0.0) {
-        const int ja = mu * 3 + other_index(mu, third_dir(mu, d, 0)), jb = mu * 3 + other_index(mu, third_dir(mu, d, 1));
-        side_acc(acc, A.c7, g, c, d, mu, Ud, A.s3 + fld(g, jb), A.t7 + fld(g, ja));
-        side_acc(acc, A.c7, g, c, d, mu, Ud, A.s3 + fld(g, ja), A.t7 + fld(g, jb));
-      }
-    }
-  } else if (A.c3 != 0.0) {
-    // 3-staples only: chain c3 M, middle U
-#pragma unroll 1
-    for (int j = 0; j < 3; j++) {
-      const int nu = other_dir(d, j);
-      staple_acc(acc, A.c3, g, c, d, nu, A.u + nu * A.ufs, A.m + d * A.mfs);
-      side_acc(acc, A.c3, g, c, d, nu, Ud, A.u + nu * A.ufs, A.m + nu * A.mfs);
+      staple_acc(acc, A.inner ? 1.0 : A.c3, g, c, d, nu, A.u + nu * A.ufs,
+                 A.inner ? A.m3 + fld(g, d * 3 + j) : A.m + d * A.mfs);
     }
   }
   if (A.lm) {
@@ -250,7 +333,7 @@ int project_u_deriv_dev(const Geom &g, const double2 *u, const double2 *x, const
 // scratch.
 int fat7_adj_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, size_t ufs, const double2 *m,
                  size_t mfs, const double2 *lm, size_t lmfs, double naik, const double2 *s3, const double2 *gm,
-                 double2 *t7, double2 *m3, double2 *d, size_t dfs, bool accumulate) {
+                 double2 *t7, double2 *m3, double2 *q, double2 *d, size_t dfs, bool accumulate) {
   AdjArgs A;
   A.g = g;
   A.u = u;
@@ -271,25 +354,33 @@ int fat7_adj_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, s
   A.c3 = c.three_staple;
   A.c7 = c.seven_staple;
   A.inner = has_inner(c) ? 1 : 0;
+  A.side = (A.inner || A.c3 != 0.0) ? 1 : 0;
+  A.q = q;
   int rc;
   if (A.inner && ((rc = staples_dev(g, u, ufs, m, mfs, t7)) ||
                   (rc = mid_dev(g, u, ufs, 0.0, nullptr, 0, c.lepage, c.five_staple, c.seven_staple, t7, m3))))
     return rc;
+  if (A.side) {
+    fat7_adj_side_kernel<<<sweep_grid(g), kSmBlock, 0, stream()>>>(A);
+    note_launch();
+  }
   fat7_adj_link_kernel<<<sweep_grid(g), kSmBlock, 0, stream()>>>(A);
   note_launch();
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
 }
 
-enum DerivSlot { kSdT7 = 40, kSdM3, kSdTmp, kSdDW, kSdIn2, kSdIn3 };
+enum DerivSlot { kSdT7 = 40, kSdM3, kSdQ, kSdTmp, kSdDW, kSdIn2, kSdIn3 };
 
-static int adj_scratch(qexstag_smear_s *s, double2 **t7, double2 **m3) {
+static int adj_scratch(qexstag_smear_s *s, double2 **t7, double2 **m3, double2 **q) {
   const size_t f = sizeof(double2) * 9 * (size_t)s->l->g.V;
-  void *a, *b;
+  void *a, *b, *c;
   int rc;
-  if ((rc = s->ws.get(kSdT7, 12 * f, &a)) || (rc = s->ws.get(kSdM3, 12 * f, &b))) return rc;
+  if ((rc = s->ws.get(kSdT7, 12 * f, &a)) || (rc = s->ws.get(kSdM3, 12 * f, &b)) || (rc = s->ws.get(kSdQ, 12 * f, &c)))
+    return rc;
   *t7 = (double2 *)a;
   *m3 = (double2 *)b;
+  *q = (double2 *)c;
   return QEXSTAG_OK;
 }
 
@@ -301,10 +392,10 @@ static int hisq_deriv_dev(qexstag_smear_s *s, const qexstag_hisq_coefs &c, const
   const Geom &geo = s->l->g;
   const size_t fs = (size_t)9 * geo.V;
   void *pv, *pw, *pd;
-  double2 *s3, *gm, *t7, *m3;
+  double2 *s3, *gm, *t7, *m3, *q;
   int rc;
   if ((rc = s->ws.get(kSmT1, field4_bytes(geo), &pv)) || (rc = s->ws.get(kSmW, field4_bytes(geo), &pw)) ||
-      (rc = s->ws.get(kSdDW, field4_bytes(geo), &pd)) || (rc = adj_scratch(s, &t7, &m3)))
+      (rc = s->ws.get(kSdDW, field4_bytes(geo), &pd)) || (rc = adj_scratch(s, &t7, &m3, &q)))
     return rc;
   double2 *v = (double2 *)pv, *w = (double2 *)pw, *dw = (double2 *)pd;
   if (!forward) {
@@ -317,14 +408,14 @@ static int hisq_deriv_dev(qexstag_smear_s *s, const qexstag_hisq_coefs &c, const
     return rc;
   }
   // second level (fat7 and Naik both of w) -> dS/dw
-  if ((rc = fat7_adj_dev(geo, c.fat7second, w, fs, cf, cfs, cl, cls, c.naik, s3, gm, t7, m3, dw, fs, false)))
+  if ((rc = fat7_adj_dev(geo, c.fat7second, w, fs, cf, cfs, cl, cls, c.naik, s3, gm, t7, m3, q, dw, fs, false)))
     return rc;
   // projectU -> dS/dv (in place)
   if ((rc = project_u_deriv_dev(geo, w, v, dw, dw, c.reunit_eps))) return rc;
   // first level: its inner fields again, then dS/dg
   if ((rc = smear_scratch(s, c.fat7first, &s3, &gm))) return rc;
   if (has_inner(c.fat7first) && (rc = fat7_inner_dev(geo, c.fat7first, g, fs, s3, gm))) return rc;
-  return fat7_adj_dev(geo, c.fat7first, g, fs, dw, fs, nullptr, 0, 0.0, s3, gm, t7, m3, d, fs, false);
+  return fat7_adj_dev(geo, c.fat7first, g, fs, dw, fs, nullptr, 0, 0.0, s3, gm, t7, m3, q, d, fs, false);
 }
 
 // F_d(x) = projectTAH(ff_d(x) U_d(x)^dag)   (fermForce's last step,
@@ -373,7 +464,7 @@ int qexstag_fat7_deriv(qexstag_smear *s, const qexstag_fat7_coefs *c, const doub
   const Geom &geo = s->l->g;
   const size_t fs = (size_t)9 * geo.V;
   const double2 *u, *m, *ul = nullptr, *lmid = nullptr, *d0;
-  double2 *d, *dl = nullptr, *s3, *gm, *t7, *m3;
+  double2 *d, *dl = nullptr, *s3, *gm, *t7, *m3, *q;
   if ((rc = smear_in(s, kSmIn0, gauge, mem, &u)) || (rc = smear_in(s, kSmIn1, mid, mem, &m)) ||
       (rc = smear_in(s, kSdIn2, deriv, mem, &d0)))
     return rc;
@@ -389,12 +480,12 @@ int qexstag_fat7_deriv(qexstag_smear *s, const qexstag_fat7_coefs *c, const doub
       dl = (double2 *)dl0;
     }
   }
-  if ((rc = smear_scratch(s, *c, &s3, &gm)) || (rc = adj_scratch(s, &t7, &m3))) return rc;
+  if ((rc = smear_scratch(s, *c, &s3, &gm)) || (rc = adj_scratch(s, &t7, &m3, &q))) return rc;
   if (has_inner(*c) && (rc = fat7_inner_dev(geo, *c, u, fs, s3, gm))) return rc;
   if (same) {
-    if ((rc = fat7_adj_dev(geo, *c, u, fs, m, fs, lmid, fs, naik, s3, gm, t7, m3, d, fs, true))) return rc;
+    if ((rc = fat7_adj_dev(geo, *c, u, fs, m, fs, lmid, fs, naik, s3, gm, t7, m3, q, d, fs, true))) return rc;
   } else {
-    if ((rc = fat7_adj_dev(geo, *c, u, fs, m, fs, nullptr, 0, 0.0, s3, gm, t7, m3, d, fs, true))) return rc;
+    if ((rc = fat7_adj_dev(geo, *c, u, fs, m, fs, nullptr, 0, 0.0, s3, gm, t7, m3, q, d, fs, true))) return rc;
     if (want_long) {
       // the Naik term alone: a level with every fat7 coefficient zero
       qexstag_fat7_coefs z;
@@ -402,7 +493,7 @@ int qexstag_fat7_deriv(qexstag_smear *s, const qexstag_fat7_coefs *c, const doub
       void *ptmp;
       if ((rc = s->ws.get(kSdTmp, field4_bytes(geo), &ptmp))) return rc;
       QS_CUDA(cudaMemsetAsync(ptmp, 0, field4_bytes(geo), stream()));
-      if ((rc = fat7_adj_dev(geo, z, ul, fs, (const double2 *)ptmp, fs, lmid, fs, naik, nullptr, nullptr, t7, m3, dl,
+      if ((rc = fat7_adj_dev(geo, z, ul, fs, (const double2 *)ptmp, fs, lmid, fs, naik, nullptr, nullptr, t7, m3, q, dl,
                              fs, true)))
         return rc;
     }

@@ -34,8 +34,10 @@ NAIK = 2 * 4 * LINK
 QEX_FLOPS_FAT7 = 61632
 # adjoint of one fat7 level: sweep A reads M and U, writes 12 T fields;
 # sweep B reads U and T, writes 12 M3 fields; sweep C reads M, U, T, M3 and
-# the forward's S and G fields and writes the derivative
-ADJ_FULL = 4 * LINK * (2 + 3) + 4 * LINK * (1 + 3 + 3) + 4 * LINK * (2 + 3 + 3 + 3 + 3 + 1)
+# the forward's S and G fields and writes 12 fields of side terms and the
+# derivative; sweep D reads M, U, T, M3 and the side terms and adds to it
+ADJ_FULL = (4 * LINK * (2 + 3) + 4 * LINK * (1 + 3 + 3) + 4 * LINK * (2 + 3 + 3 + 3 + 3 + 3 + 1)
+            + 4 * LINK * (2 + 3 + 3 + 3 + 2))
 ADJ_NAIK = 4 * LINK  # the long-link chain, read once more by sweep C
 PROJECT_DERIV = 4 * LINK * 4  # reads v, w, the chain; writes the result
 

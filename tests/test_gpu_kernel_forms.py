@@ -6,6 +6,7 @@ import pytest
 
 from oracle import oracle as O
 from qex_b200 import fields as F
+from qex_b200 import smear as SM
 from qex_b200 import stag as S
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +34,22 @@ def test_half_sweep_forms(cuda, dims, naik):
     s.stagD2ee(r, S.to_device_vector(x), 0.01)
     o.stagD2ee(ro, x, 0.01)
     assert rel(S.to_host_vector(r), ro) < 1e-13
+
+
+# smearing sweeps: blocks of 64 half sites of both parities; 720 half sites
+# are 11 1/4 of them and 22 1/2 warps (tolerances as for the other shapes)
+@pytest.mark.parametrize("coef", [[0.3, 0.2, -0.1, 0.05, 0.07], [0.4, 0.2, 0.0, 0.0, 0.0], [0.3, 0.2, -0.1, 0.0, 0.0],
+                                  [0.3, 0.0, 0.0, 0.05, 0.0], [0.3, 0.2, 0.0, 0.0, 0.07], [0.5, 0.0, 0.0, 0.0, 0.0]])
+def test_smearing_sweep_remainders(cuda, coef):
+    dims = (4, 6, 6, 10)
+    V = F.volume(dims)
+    g = O.apply_phases(dims, F.gauge_warm(dims, 0.5, 6))
+    rng = np.random.default_rng(7)
+    ch, d0 = (rng.standard_normal((4, V, 3, 3)) + 1j * rng.standard_normal((4, V, 3, 3)) for _ in range(2))
+    sm, c = SM.Smear(S.Layout(dims)), SM.Fat7lCoefs(*coef)
+    fl = np.empty_like(g)
+    sm.makeImpLinks(fl, g, c)
+    assert rel(fl, O.fat7(dims, coef, g)) < 1e-12
+    d = d0.copy()
+    sm.fat7Deriv(d, g, ch, c)
+    assert rel(d, d0 + O.fat7_deriv(dims, coef, g, ch)[0]) < 1e-12
