@@ -284,9 +284,9 @@ long long launch_count();
 // launch a kernel that begins with pdl_wait() with programmatic stream
 // serialisation on the library's stream
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, Args... args) {
+inline cudaError_t launch_pdl2(void (*kern)(KArgs...), dim3 grid, int block, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = stream();
@@ -296,6 +296,10 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, Args.
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, ((KArgs)args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, Args... args) {
+  return launch_pdl2(kern, dim3((unsigned)grid), block, args...);
 }
 
 inline int grid_for(long n, int block = kBlock, int per_sm = 8) {

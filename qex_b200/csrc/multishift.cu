@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "lib.cuh"
@@ -25,9 +26,10 @@ constexpr int kMaxRhs = 8;
 
 struct CgmState {
   int itn, maxits, done, dropping;
-  int nshift, nrhs, pad0, pad1;
-  int live[kMaxRhs];  // right-hand side still iterating this iteration
-  int cont[kMaxRhs];  // continuing after this iteration
+  int nshift, nrhs;
+  int last;           // the iteration that ended the last live right-hand side
+  int pad0;
+  int live[kMaxRhs];  // right-hand side still iterating
   double r2i[kMaxRhs], pAp[kMaxRhs], alpha[kMaxRhs], beta[kMaxRhs];
   double alphaim1[kMaxRhs], betaim1[kMaxRhs], r2stop[kMaxRhs], b2[kMaxRhs];
   double sg[kMaxShift];
@@ -36,37 +38,94 @@ struct CgmState {
   int dox[kMaxRhs][kMaxShift], dop[kMaxRhs][kMaxShift], active[kMaxRhs][kMaxShift];
 };
 
-// vectors of the solve: [nrhs][3][nh] (r, Ap, t) and [nrhs][nshift][3][nh]
-// (x, p); element type double2 (FP64) or float2 (FP32)
+// Element types of the solve's vectors: double2 or float2, one right-hand
+// side, or float4, a pair of them as (re_0, re_1, im_0, im_1), which one
+// 16-byte load brings and one FP32x2 operation advances.
+template <class VT>
+struct Lanes {
+  static constexpr int n = 1;
+};
+template <>
+struct Lanes<float4> {
+  static constexpr int n = 2;
+};
+__device__ __forceinline__ double2 &lane(double2 &v, int) { return v; }
+__device__ __forceinline__ float2 &lane(float2 &v, int) { return v; }
+struct Lane4 {
+  float &x, &y;
+};
+__device__ __forceinline__ Lane4 lane(float4 &v, int q) { return q == 0 ? Lane4{v.x, v.z} : Lane4{v.y, v.w}; }
+
+// vectors of the solve: [nrhs / n][3][nh] (r, Ap, t) and [nrhs / n][nshift][3][nh]
+// (x, p), n right-hand sides to an element (an odd last one has a zero partner)
 template <class VT>
 struct CgmVecs {
   VT *r, *ap, *t, *x, *p;
-  int nh, nshift, nrhs;
+  int nh, nshift, nvec;
   __host__ __device__ size_t rhs_off(int j) const { return (size_t)j * 3 * nh; }
   __host__ __device__ size_t xs_off(int j, int k) const { return ((size_t)j * nshift + k) * 3 * nh; }
 };
 
+// The sum over the grid of one double per right-hand side, from each warp's
+// part: warps hold a part of right-hand side j in lane 0 and have stored it at
+// partials[j * stride + slot]; the last block's warp j adds them in slot order
+// of its lanes.  True in the last block, where sum is the total of right-hand
+// side (warp) in every lane of that warp.  stride slots, blocks of kBlock
+// threads (kMaxRhs warps).
+__device__ __forceinline__ bool rhs_reduce(int nrhs, const double *partials, int stride, unsigned *ticket,
+                                           unsigned nblocks, double &sum) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == nblocks - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double s = 0.0;
+  if (w < nrhs)
+    for (int i = l; i < stride; i += 32) s += __ldcg(partials + (size_t)w * stride + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  sum = s;
+  if (threadIdx.x == 0) *ticket = 0u;
+  return true;
+}
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // ---------------------------------------------------------------------------
-// FP32 multi-right-hand-side Dslash: a block is kMrhsGroups warp-uniform
-// groups of kMrhsSites sites; group q applies the operator to right-hand
-// sides q*kMrhsPer .. q*kMrhsPer+kMrhsPer-1 of its sites.  Every group loads
-// the same links, so each link comes from HBM once per site and from L1 for
-// the other groups, while each right-hand side's vector loads stay
-// coalesced across the warp.
+// FP32 multi-right-hand-side Dslash on pairs of right-hand sides.  A block is
+// eight warps: a set of 32 sites takes 4 G of them, G = 1 or 2 groups of NP
+// pairs times the four directions, and a block holds 2 / G sets.  Warp
+// (mu, group) forms the direction's hops, forward and backward, fat and long,
+// for its pairs: every link is read from HBM once and from L1 by the other
+// group, a vector load brings both right-hand sides of a pair, and the sums
+// run in FP32x2 arithmetic with the link's parts broadcast.  The four
+// directions' sums meet in shared memory.
+//
+// Bound by the latency of the gathers through L2 and by how many sites the
+// register file keeps in flight: at 16^4 fat+Naik with 8 right-hand sides 24 us
+// (first sweep) and 32 us (second, with the sums), as a thread that walks all
+// hops of 4 right-hand sides took; one pair a thread in 512-thread blocks took
+// 27 and 39 us at 64 registers, 35 and 47 at 128.
 // ---------------------------------------------------------------------------
 
-constexpr int kMrhsPer = 4;                       // right-hand sides per thread
-constexpr int kMrhsGroups = kMaxRhs / kMrhsPer;   // 2
-constexpr int kMrhsSites = kBlock / kMrhsGroups;  // 128 sites per block step
+constexpr int kMrhsSites = 32;  // sites of a set
 
 struct MrhsArgs {
   Geom g;
-  int po, nr;
+  int po, nr, npair;
   LoLinks L;
-  const float2 *xin;  // [nr][3][nh]
-  const float2 *xs;   // [nr][3][nh] same-site operand (INIT)
-  float2 *out;        // [nr][3][nh]
-  size_t irs, srs, ors;  // right-hand-side strides of xin, xs, out
+  const float4 *xin;  // [npair][3][nh]
+  const float4 *xs;   // [npair][3][nh] same-site operand (INIT)
+  float4 *out;        // [npair][3][nh]
+  size_t irs, srs, ors;  // pair strides of xin, xs, out
   int nh;
   float b;
   const CgmState *st;
@@ -75,8 +134,19 @@ struct MrhsArgs {
   unsigned *ticket;
 };
 
-template <int NL, int HOP, int INIT, int RED, int R12>
+// (re, im) += (ar, ai) (vr, vi) for both right-hand sides of a pair, nai = -ai
+__device__ __forceinline__ void pair_mac(float2 &re, float2 &im, float ar, float ai, float nai, float2 vr, float2 vi) {
+  const float2 ar2 = make_float2(ar, ar), ai2 = make_float2(ai, ai), nai2 = make_float2(nai, nai);
+  re = __ffma2_rn(ar2, vr, re);
+  re = __ffma2_rn(nai2, vi, re);
+  im = __ffma2_rn(ar2, vi, im);
+  im = __ffma2_rn(ai2, vr, im);
+}
+
+template <int NL, int HOP, int INIT, int RED, int R12, int NP, int G>
 __global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A) {
+  constexpr int kSets = 2 / G;
+  __shared__ float4 part[kSets][4][G * NP][3][kMrhsSites];
   pdl_wait();
   if (A.st->done) return;
   const Geom &g = A.g;
@@ -84,103 +154,121 @@ __global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A
   const size_t V = (size_t)g.V;
   const size_t in_base = (size_t)(1 - A.po) * nh;
   const size_t out_base = (size_t)A.po * nh;
-  const int grp = threadIdx.x / kMrhsSites;
-  const int j0 = grp * kMrhsPer;
-  double dot[kMrhsPer];
+  const int lane_ = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int mu = w & 3, grp = G == 2 ? w >> 2 : 0, set = G == 2 ? 0 : w >> 2;
+  // after the meeting: warp w adds pair fp of set fset
+  const int fset = w / (G * NP), fp = w - fset * (G * NP);
+  const bool adds = fset < kSets && fp < A.npair;
+  double dot[2] = {0.0, 0.0};
+  for (int k0 = blockIdx.x * (kMrhsSites * kSets); k0 < nh; k0 += gridDim.x * (kMrhsSites * kSets)) {
+    {
+      const int kk = k0 + set * kMrhsSites + lane_;
+      const int k = min(kk, nh - 1);
+      int x[4], lex;
+      site_coords(g, A.po, k, x, lex);
+      float2 re[NP][3], im[NP][3];
 #pragma unroll
-  for (int q = 0; q < kMrhsPer; q++) dot[q] = 0.0;
-  for (int k = blockIdx.x * kMrhsSites + (threadIdx.x % kMrhsSites); k < nh; k += gridDim.x * kMrhsSites) {
-    if (j0 >= A.nr) break;
-    int x[4], lex;
-    site_coords(g, A.po, k, x, lex);
-    float2 acc[kMrhsPer][3];
+      for (int q = 0; q < NP; q++)
 #pragma unroll
-    for (int q = 0; q < kMrhsPer; q++)
+        for (int c = 0; c < 3; c++) re[q][c] = im[q][c] = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int c = 0; c < 3; c++) acc[q][c] = make_float2(0.f, 0.f);
+      for (int h = 0; h < NL / 4; h++) {
+        const int len = h == 0 ? 1 : 3;
 #pragma unroll
-    for (int l = 0; l < NL; l++) {
-      const int mu = Hop<NL>::mu(l), len = Hop<NL>::len(l);
-      const bool is_long = (NL == 8) && (l & 1);
-      const int f = (NL == 8) ? (l >> 1) : l;
-      const int jf = nbr_half(g, x, lex, mu, len);
-      const int jb = nbr_half(g, x, lex, mu, -len);
-      float2 uf[9], ub[9];
-      if (is_long && R12) {
-        load_long12<kF32>(A.L, f, out_base + k, V, long_sign_fwd(g, x, mu), uf);
-        load_long12<kF32>(A.L, f, in_base + jb, V, long_sign_bck(g, x, mu), ub);
-      } else if (is_long) {
-        load_link18<kF32>(A.L.f32_long, A.L.f32_long_tail, nullptr, nullptr, f, out_base + k, V, uf);
-        load_link18<kF32>(A.L.f32_long, A.L.f32_long_tail, nullptr, nullptr, f, in_base + jb, V, ub);
-      } else {
-        load_link18<kF32>(A.L.f32_fat, A.L.f32_fat_tail, nullptr, nullptr, f, out_base + k, V, uf);
-        load_link18<kF32>(A.L.f32_fat, A.L.f32_fat_tail, nullptr, nullptr, f, in_base + jb, V, ub);
-      }
+        for (int dir = 0; dir < 2; dir++) {
+          const int jn = (lex + lex_step(g, x, mu, dir ? -len : len)) >> 1;
+          const size_t us = dir ? in_base + jn : out_base + k;
+          float2 u[9];
+          if (h == 1 && R12)
+            load_long12<kF32>(A.L, mu, us, V, dir ? long_sign_bck(g, x, mu) : long_sign_fwd(g, x, mu), u);
+          else if (h == 1)
+            load_link18<kF32>(A.L.f32_long, A.L.f32_long_tail, nullptr, nullptr, mu, us, V, u);
+          else
+            load_link18<kF32>(A.L.f32_fat, A.L.f32_fat_tail, nullptr, nullptr, mu, us, V, u);
 #pragma unroll
-      for (int q = 0; q < kMrhsPer; q++) {
-        const int j = j0 + q;
-        if (j < A.nr) {
-          const float2 *xj = A.xin + (size_t)j * A.irs;
-          float2 v[3], w[3];
+          for (int q = 0; q < NP; q++) {
+            const int p = grp * NP + q;
+            if (p < A.npair) {
+              const float4 *xp = A.xin + (size_t)p * A.irs + jn;
+              float4 v[3];
 #pragma unroll
-          for (int c = 0; c < 3; c++) {
-            v[c] = ldg(xj + (size_t)c * nh + jf);
-            w[c] = ldg(xj + (size_t)c * nh + jb);
-          }
+              for (int c = 0; c < 3; c++) v[c] = ldg(xp + (size_t)c * nh);
 #pragma unroll
-          for (int i = 0; i < 3; i++) {
-            float2 t = make_float2(0.f, 0.f), u = make_float2(0.f, 0.f);
+              for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-              t = cmadd(t, uf[3 * i + c], v[c]);
-              u = cjmadd(u, ub[3 * c + i], w[c]);
-            }
-            if (HOP > 0) {
-              acc[q][i].x += t.x - u.x;
-              acc[q][i].y += t.y - u.y;
-            } else {
-              acc[q][i].x -= t.x - u.x;
-              acc[q][i].y -= t.y - u.y;
+                for (int c = 0; c < 3; c++) {
+                  const float2 vr = make_float2(v[c].x, v[c].y), vi = make_float2(v[c].z, v[c].w);
+                  // forward + U_ic v_c; backward - conj(U_ci) v_c
+                  if (dir == 0)
+                    pair_mac(re[q][i], im[q][i], u[3 * i + c].x, u[3 * i + c].y, -u[3 * i + c].y, vr, vi);
+                  else
+                    pair_mac(re[q][i], im[q][i], -u[3 * c + i].x, u[3 * c + i].y, -u[3 * c + i].y, vr, vi);
+                }
             }
           }
         }
       }
+#pragma unroll
+      for (int q = 0; q < NP; q++)
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          part[set][mu][grp * NP + q][c][lane_] = make_float4(re[q][c].x, re[q][c].y, im[q][c].x, im[q][c].y);
     }
+    __syncthreads();
+    const int k = k0 + fset * kMrhsSites + lane_;
+    if (adds && k < nh) {
+      float d0 = 0.f, d1 = 0.f;
 #pragma unroll
-    for (int q = 0; q < kMrhsPer; q++) {
-      const int j = j0 + q;
-      if (j < A.nr) {
-        float2 *oj = A.out + (size_t)j * A.ors;
-        float d = 0.f;
+      for (int c = 0; c < 3; c++) {
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          float2 o = acc[q][c];
-          if (INIT) {
-            float2 s = __ldcg(A.xs + (size_t)j * A.srs + (size_t)c * nh + k);
-            o.x = fmaf(A.b, s.x, o.x);
-            o.y = fmaf(A.b, s.y, o.y);
-            if (RED) d += s.x * o.x + s.y * o.y;
-          }
-          oj[(size_t)c * nh + k] = o;
+        for (int m = 0; m < 4; m++) {
+          const float4 t = part[fset][m][fp][c][lane_];
+          o.x += t.x;
+          o.y += t.y;
+          o.z += t.z;
+          o.w += t.w;
         }
-        if (RED) dot[q] += (double)d;
+        if (HOP < 0) o = make_float4(-o.x, -o.y, -o.z, -o.w);
+        if (INIT) {
+          const float4 s = __ldcg(A.xs + (size_t)fp * A.srs + (size_t)c * nh + k);
+          o.x = fmaf(A.b, s.x, o.x);
+          o.y = fmaf(A.b, s.y, o.y);
+          o.z = fmaf(A.b, s.z, o.z);
+          o.w = fmaf(A.b, s.w, o.w);
+          if (RED) {
+            d0 = fmaf(s.x, o.x, fmaf(s.z, o.z, d0));
+            d1 = fmaf(s.y, o.y, fmaf(s.w, o.w, d1));
+          }
+        }
+        A.out[(size_t)fp * A.ors + (size_t)c * nh + k] = o;
+      }
+      if (RED) {
+        dot[0] += (double)d0;
+        dot[1] += (double)d1;
       }
     }
+    __syncthreads();
   }
   if (RED) {
-    // each right-hand side's sum from its group's threads (static indices)
-    double all[kMaxRhs];
-#pragma unroll
-    for (int j = 0; j < kMaxRhs; j++) all[j] = (j / kMrhsPer == grp) ? dot[j % kMrhsPer] : 0.0;
-    double s[kMaxRhs];
-    if (grid_reduce<kMaxRhs>(all, A.partials, A.ticket, s) && threadIdx.x == 0)
-      for (int j = 0; j < A.nr; j++) A.wst->pAp[j] = s[j];
+    const int stride = gridDim.x * kSets;
+    dot[0] = warp_sum(dot[0]);
+    dot[1] = warp_sum(dot[1]);
+    if (adds && lane_ == 0) {
+      const int slot = blockIdx.x * kSets + fset;
+      A.partials[(size_t)(2 * fp) * stride + slot] = dot[0];
+      if (2 * fp + 1 < A.nr) A.partials[(size_t)(2 * fp + 1) * stride + slot] = dot[1];
+    }
+    double s;
+    if (rhs_reduce(A.nr, A.partials, stride, A.ticket, gridDim.x, s) && w < A.nr && lane_ == 0) A.wst->pAp[w] = s;
   }
 }
 
-template <int NL, int R12>
-static void mrhs_pair(MrhsArgs A, int par, const float2 *p, size_t prs, float2 *t, float2 *ap, float b4m2,
-                      int grid) {
+template <int NL, int R12, int NP, int G>
+static void mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
+  const int sets = 2 / G, per = kMrhsSites * sets;
+  // slots of the reduction: 8 right-hand sides share red_partials
+  const int grid = std::min({(A.nh + per - 1) / per, num_sms() * 6, kMaxRedBlocks / sets});
   const size_t vs = (size_t)3 * A.nh;
   A.po = 1 - par;
   A.xin = p;
@@ -190,7 +278,7 @@ static void mrhs_pair(MrhsArgs A, int par, const float2 *p, size_t prs, float2 *
   A.out = t;
   A.ors = vs;
   A.b = 0.f;
-  launch_pdl(dslash_mrhs_kernel<NL, 1, 0, 0, R12>, grid, kBlock, A);
+  launch_pdl(dslash_mrhs_kernel<NL, 1, 0, 0, R12, NP, G>, grid, kBlock, A);
   A.po = par;
   A.xin = t;
   A.irs = vs;
@@ -199,122 +287,143 @@ static void mrhs_pair(MrhsArgs A, int par, const float2 *p, size_t prs, float2 *
   A.out = ap;
   A.ors = vs;
   A.b = b4m2;
-  launch_pdl(dslash_mrhs_kernel<NL, -1, 1, 1, R12>, grid, kBlock, A);
+  launch_pdl(dslash_mrhs_kernel<NL, -1, 1, 1, R12, NP, G>, grid, kBlock, A);
   note_launch(2);
 }
 
-// p_j at p + j*prs; t_j, ap_j at j*3*nh
-static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float2 *p, size_t prs, float2 *t,
-                      float2 *ap, double m2, CgmState *st) {
+template <int NL, int R12>
+static void mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
+  if (A.npair == 1)
+    mrhs_pair<NL, R12, 1, 1>(A, par, p, prs, t, ap, b4m2);
+  else if (A.npair == 2)
+    mrhs_pair<NL, R12, 2, 1>(A, par, p, prs, t, ap, b4m2);
+  else
+    mrhs_pair<NL, R12, 2, 2>(A, par, p, prs, t, ap, b4m2);
+}
+
+// pair j of p at p + j*prs; of t and ap at j*3*nh
+static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p, size_t prs, float4 *t,
+                      float4 *ap, double m2, CgmState *st) {
   const Geom &geo = g->l->g;
   MrhsArgs A;
   A.g = geo;
   A.nr = nr;
+  A.npair = (nr + 1) / 2;
   A.L = lo_links(g->low, kF32);
   A.nh = geo.nh;
   A.st = st;
   A.wst = st;
   A.partials = red_partials();
   A.ticket = red_tickets();
-  // blocks step over kMrhsSites sites; at most kMaxRedBlocks*8/kMaxRhs for the reduction
-  int grid = (int)std::min<long>(((long)geo.nh + kMrhsSites - 1) / kMrhsSites, (long)num_sms() * 4);
-  if (grid * kMaxRhs > kMaxRedBlocks * 8) grid = kMaxRedBlocks * 8 / kMaxRhs;
-  if (grid < 1) grid = 1;
   const float b4 = (float)(4.0 * m2);
   if (g->nl == 8) {
     if (g->low.recon12)
-      mrhs_pair<8, 1>(A, par, p, prs, t, ap, b4, grid);
+      mrhs_pairs<8, 1>(A, par, p, prs, t, ap, b4);
     else
-      mrhs_pair<8, 0>(A, par, p, prs, t, ap, b4, grid);
+      mrhs_pairs<8, 0>(A, par, p, prs, t, ap, b4);
   } else {
-    mrhs_pair<4, 0>(A, par, p, prs, t, ap, b4, grid);
+    mrhs_pairs<4, 0>(A, par, p, prs, t, ap, b4);
   }
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
 }
 
 // ---------------------------------------------------------------------------
-// CG-M iteration kernels (element type VT)
+// CG-M iteration kernels (element type VT); block row y works on element y of
+// the vectors, so that every right-hand side has its own threads
 // ---------------------------------------------------------------------------
 
-__global__ void cgm_alpha_kernel(CgmState *st) {
-  if (st->done) return;
-  for (int j = 0; j < st->nrhs; j++) {
-    double pAp = st->pAp[j];
-    st->alpha[j] = (pAp != 0.0) ? st->r2i[j] / pAp : 0.0;
-  }
-  st->itn += 1;
+template <class L1, class L2>
+__device__ __forceinline__ void axpy2(L1 &&y, double a, L2 &&x) {
+  using R = std::remove_reference_t<decltype(y.x)>;
+  y.x = fma((R)a, x.x, y.x);
+  y.y = fma((R)a, x.y, y.y);
 }
 
-template <class VT>
-__device__ __forceinline__ VT vload(const VT *p) { return *p; }
-
-__device__ __forceinline__ void axpy2(double2 &y, double a, double2 x) {
-  y.x = fma(a, x.x, y.x);
-  y.y = fma(a, x.y, y.y);
-}
-__device__ __forceinline__ void axpy2(float2 &y, double a, float2 x) {
-  y.x = fmaf((float)a, x.x, y.x);
-  y.y = fmaf((float)a, x.y, y.y);
-}
-
-// cgm.nim:157-184 for shift 0: r -= alpha Ap; x0 += alpha p0; |r|^2; then the
-// zeta recurrences of every other shift (cgm.nim:187-200)
+// cgm.nim:157-184 for shift 0: r -= alpha Ap; x0 += alpha p0; |r|^2; then, in
+// the last block, the zeta recurrences of every other shift (cgm.nim:187-200):
+// warp j, lane k for shift k of right-hand side j.  alpha = r2 / <p, Ap> comes
+// from the sums the operator left.  (One thread that walked the 8 x 6 scalars
+// one by one, and two one-thread kernels around it for alpha and the end
+// test, took 25 us an iteration at 16^4; this takes 11.5.  Whole 8-system,
+// 6-shift solve: 238 -> 181 ms.)
 template <class VT>
 __global__ void __launch_bounds__(kBlock) cgm_update1_kernel(CgmVecs<VT> v, CgmState *st, double *partials,
                                                             unsigned *ticket) {
+  pdl_wait();
   if (st->done) return;
-  const int nh = v.nh;
-  double s[kMaxRhs];
+  constexpr int n = Lanes<VT>::n;
+  const int nh = v.nh, e = blockIdx.y;
+  __shared__ double sh[n * 32];
+  double a[n], s[n];
+  bool any = false;
 #pragma unroll
-  for (int j = 0; j < kMaxRhs; j++) s[j] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
+  for (int q = 0; q < n; q++) {
+    const int j = e * n + q;
+    const bool on = j < st->nrhs && st->live[j] != 0;
+    const double pAp = on ? st->pAp[j] : 0.0;
+    a[q] = pAp != 0.0 ? st->r2i[j] / pAp : 0.0;
+    s[q] = 0.0;
+    any |= on;
+  }
+  if (any) {
+    VT *r = v.r + v.rhs_off(e);
+    const VT *ap = v.ap + v.rhs_off(e);
+    VT *x0 = v.x + v.xs_off(e, 0);
+    const VT *p0 = v.p + v.xs_off(e, 0);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
+      VT rv[3], xv[3], av[3], pv[3];
 #pragma unroll
-    for (int j = 0; j < kMaxRhs; j++) {
-      if (j < v.nrhs && st->live[j]) {
-        const double a = st->alpha[j];
-        VT *r = v.r + v.rhs_off(j);
-        const VT *ap = v.ap + v.rhs_off(j);
-        VT *x0 = v.x + v.xs_off(j, 0);
-        const VT *p0 = v.p + v.xs_off(j, 0);
-        double acc = 0.0;
+      for (int c = 0; c < 3; c++) {
+        const size_t o = (size_t)c * nh + i;
+        rv[c] = r[o];
+        av[c] = ap[o];
+        xv[c] = x0[o];
+        pv[c] = p0[o];
+      }
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const size_t o = (size_t)c * nh + i;
-          VT rv = r[o], xv = x0[o];
-          axpy2(rv, -a, ap[o]);
-          axpy2(xv, a, p0[o]);
-          r[o] = rv;
-          x0[o] = xv;
-          acc += (double)rv.x * rv.x + (double)rv.y * rv.y;
+      for (int c = 0; c < 3; c++) {
+        const size_t o = (size_t)c * nh + i;
+#pragma unroll
+        for (int q = 0; q < n; q++) {
+          axpy2(lane(rv[c], q), -a[q], lane(av[c], q));
+          axpy2(lane(xv[c], q), a[q], lane(pv[c], q));
+          s[q] += (double)lane(rv[c], q).x * lane(rv[c], q).x + (double)lane(rv[c], q).y * lane(rv[c], q).y;
         }
-        s[j] += acc;
+        r[o] = rv[c];
+        x0[o] = xv[c];
       }
     }
   }
-  double tot[kMaxRhs];
-  if (!(grid_reduce<kMaxRhs>(s, partials, ticket, tot) && threadIdx.x == 0)) return;
-  for (int j = 0; j < st->nrhs; j++) {
-    if (!st->live[j]) continue;
-    const double alpha = st->alpha[j], r2i = st->r2i[j];
-    const double r2ip1 = tot[j];
-    const double beta = (r2i != 0.0) ? r2ip1 / r2i : 0.0;
-    const bool cont = (st->itn < st->maxits) && (r2ip1 > st->r2stop[j]);
-    st->beta[j] = beta;
-    for (int k = 1; k < st->nshift; k++) {
-      if (!st->active[j][k]) {
-        st->dox[j][k] = st->dop[j][k] = 0;
-        continue;
-      }
+  block_sum<n>(s, sh);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < n; q++)
+      if (e * n + q < st->nrhs) partials[(size_t)(e * n + q) * gridDim.x + blockIdx.x] = s[q];
+  }
+  double r2ip1;
+  const int nrhs = st->nrhs, nshift = st->nshift;
+  if (!rhs_reduce(nrhs, partials, gridDim.x, ticket, gridDim.x * gridDim.y, r2ip1)) return;
+  const int j = threadIdx.x >> 5, k = threadIdx.x & 31;
+  const int itn = st->itn + 1;
+  int cont = 0;
+  if (j < nrhs) {
+    const bool live = st->live[j] != 0;
+    const double pAp = st->pAp[j], r2i = st->r2i[j];
+    const double alpha = pAp != 0.0 ? r2i / pAp : 0.0;
+    const double beta = r2i != 0.0 ? r2ip1 / r2i : 0.0;
+    cont = live && itn < st->maxits && r2ip1 > st->r2stop[j];
+    int dox = 0, dop = 0;
+    if (live && k > 0 && k < nshift && st->active[j][k]) {
       const double zi = st->zi[j][k], zim1 = st->zim1[j][k], sg = st->sg[k];
       double zip1d = alpha * st->betaim1[j] * (zim1 - zi);
       zip1d += zim1 * st->alphaim1[j] * (1.0 + sg * alpha);
       const double zip1 = (zip1d != 0.0) ? zi * zim1 * st->alphaim1[j] / zip1d : 0.0;
       const double zr = (zi != 0.0) ? zip1 / zi : 0.0;
       st->cx[j][k] = alpha * zr;
-      st->dox[j][k] = 1;
-      st->dop[j][k] = cont ? 1 : 0;
+      dox = 1;
       if (cont) {
+        dop = 1;
         st->cr[j][k] = zip1;
         st->cp[j][k] = beta * zr * zr;
         st->zim1[j][k] = zi;
@@ -323,72 +432,90 @@ __global__ void __launch_bounds__(kBlock) cgm_update1_kernel(CgmVecs<VT> v, CgmS
         if (st->dropping && zip1 * zip1 * r2ip1 <= st->r2stop[j]) st->active[j][k] = 0;
       }
     }
-    st->alphaim1[j] = alpha;
-    st->betaim1[j] = beta;
-    st->r2i[j] = r2ip1;
-    st->cont[j] = cont ? 1 : 0;
+    if (k < nshift) {
+      st->dox[j][k] = dox;
+      st->dop[j][k] = k == 0 ? cont : dop;
+    }
+    __syncwarp();
+    if (k == 0 && live) {
+      st->beta[j] = beta;
+      st->alphaim1[j] = alpha;
+      st->betaim1[j] = beta;
+      st->r2i[j] = r2ip1;
+      st->live[j] = cont;
+    }
   }
-}
-
-// p0 = r + beta p0; x_k += cx p_k; p_k = cr r + cp p_k
-template <class VT>
-__global__ void cgm_update2_kernel(CgmVecs<VT> v, const CgmState *st) {
-  if (st->done) return;
-  const int nh = v.nh;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
-    for (int j = 0; j < v.nrhs; j++) {
-      if (!st->live[j]) continue;
-      const VT *r = v.r + v.rhs_off(j);
-      VT rv[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) rv[c] = r[(size_t)c * nh + i];
-      if (st->cont[j]) {
-        VT *p0 = v.p + v.xs_off(j, 0);
-        const double b = st->beta[j];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const size_t o = (size_t)c * nh + i;
-          VT pv = p0[o];
-          VT q = rv[c];
-          axpy2(q, b, pv);
-          p0[o] = q;
-        }
-      }
-      for (int k = 1; k < v.nshift; k++) {
-        if (!st->dox[j][k]) continue;
-        VT *xk = v.x + v.xs_off(j, k);
-        VT *pk = v.p + v.xs_off(j, k);
-        const double cx = st->cx[j][k];
-        const bool dp = st->dop[j][k];
-        const double cr = st->cr[j][k], cp = st->cp[j][k];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const size_t o = (size_t)c * nh + i;
-          VT pv = pk[o], xv = xk[o];
-          axpy2(xv, cx, pv);
-          xk[o] = xv;
-          if (dp) {
-            VT q;
-            q.x = 0;
-            q.y = 0;
-            axpy2(q, cr, rv[c]);
-            axpy2(q, cp, pv);
-            pk[o] = q;
-          }
-        }
-      }
+  const int more = __syncthreads_or(cont);
+  if (threadIdx.x == 0) {
+    st->itn = itn;
+    if (!more) {
+      st->last = itn;
+      st->done = 1;
     }
   }
 }
 
-__global__ void cgm_finish_kernel(CgmState *st) {
-  if (st->done) return;
-  int any = 0;
-  for (int j = 0; j < st->nrhs; j++) {
-    st->live[j] = st->cont[j];
-    any |= st->cont[j];
+// p0 = r + beta p0; x_k += cx p_k; p_k = cr r + cp p_k, of iteration it (the
+// last one included: its x_k still move when update1 has ended the solve)
+template <class VT>
+__global__ void __launch_bounds__(kBlock) cgm_update2_kernel(CgmVecs<VT> v, const CgmState *st, int it) {
+  pdl_wait();
+  if (st->done && it > st->last) return;
+  constexpr int n = Lanes<VT>::n;
+  const int nh = v.nh, e = blockIdx.y, nshift = v.nshift;
+  __shared__ double cx[n][kMaxShift], cr[n][kMaxShift], cp[n][kMaxShift];
+  __shared__ int moves[kMaxShift], turns[n][kMaxShift];
+  for (int t = threadIdx.x; t < nshift; t += blockDim.x) {
+    int mv = 0;
+#pragma unroll
+    for (int q = 0; q < n; q++) {
+      const int j = e * n + q;
+      const bool on = j < st->nrhs;
+      const int dox = on ? st->dox[j][t] : 0, dop = on ? st->dop[j][t] : 0;
+      cx[q][t] = dox ? st->cx[j][t] : 0.0;
+      cr[q][t] = t == 0 ? 1.0 : dop ? st->cr[j][t] : 0.0;
+      cp[q][t] = dop ? (t == 0 ? st->beta[j] : st->cp[j][t]) : 0.0;
+      turns[q][t] = dop;
+      mv |= dox | dop;
+    }
+    moves[t] = mv;
   }
-  if (!any) st->done = 1;
+  __syncthreads();
+  const VT *r = v.r + v.rhs_off(e);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
+    VT rv[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) rv[c] = r[(size_t)c * nh + i];
+    for (int k = 0; k < nshift; k++) {
+      if (!moves[k]) continue;
+      VT *xk = v.x + v.xs_off(e, k);
+      VT *pk = v.p + v.xs_off(e, k);
+      VT pv[3], xv[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        pv[c] = pk[(size_t)c * nh + i];
+        if (k > 0) xv[c] = xk[(size_t)c * nh + i];
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+#pragma unroll
+        for (int q = 0; q < n; q++) {
+          if (k > 0) axpy2(lane(xv[c], q), cx[q][k], lane(pv[c], q));
+          if (turns[q][k]) {
+            VT z = rv[c];
+            lane(z, q).x = 0;
+            lane(z, q).y = 0;
+            axpy2(lane(z, q), cr[q][k], lane(rv[c], q));
+            axpy2(lane(z, q), cp[q][k], lane(pv[c], q));
+            lane(pv[c], q).x = lane(z, q).x;
+            lane(pv[c], q).y = lane(z, q).y;
+          }
+        }
+        if (k > 0) xk[(size_t)c * nh + i] = xv[c];
+        pk[(size_t)c * nh + i] = pv[c];
+      }
+    }
+  }
 }
 
 // initial state: r = b, x = 0, p_k = r; |b|^2 per right-hand side
@@ -396,64 +523,73 @@ template <class VT>
 __global__ void __launch_bounds__(kBlock) cgm_init_kernel(CgmVecs<VT> v, const double2 *const *b, int bstride,
                                                          CgmState *st, double *partials, unsigned *ticket,
                                                          double r2req) {
-  const int nh = v.nh;
-  double s[kMaxRhs];
+  constexpr int n = Lanes<VT>::n;
+  const int nh = v.nh, e = blockIdx.y, nrhs = st->nrhs;
+  __shared__ double sh[n * 32];
+  double s[n];
 #pragma unroll
-  for (int j = 0; j < kMaxRhs; j++) s[j] = 0.0;
+  for (int q = 0; q < n; q++) s[q] = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
+    for (int c = 0; c < 3; c++) {
+      VT rv{}, z{};
 #pragma unroll
-    for (int j = 0; j < kMaxRhs; j++) {
-      if (j < v.nrhs) {
-        const double2 *bj = b[j];
-        double acc = 0.0;
-        for (int c = 0; c < 3; c++) {
-          double2 bv = bj[(size_t)c * bstride + i];
-          VT rv;
-          rv.x = bv.x;
-          rv.y = bv.y;
-          v.r[v.rhs_off(j) + (size_t)c * nh + i] = rv;
-          VT z;
-          z.x = 0;
-          z.y = 0;
-          for (int k = 0; k < v.nshift; k++) {
-            v.x[v.xs_off(j, k) + (size_t)c * nh + i] = z;
-            v.p[v.xs_off(j, k) + (size_t)c * nh + i] = rv;
-          }
-          acc += bv.x * bv.x + bv.y * bv.y;
+      for (int q = 0; q < n; q++) {
+        const int j = e * n + q;
+        if (j < nrhs) {
+          const double2 bv = b[j][(size_t)c * bstride + i];
+          lane(rv, q).x = bv.x;
+          lane(rv, q).y = bv.y;
+          s[q] += bv.x * bv.x + bv.y * bv.y;
         }
-        s[j] += acc;
+      }
+      v.r[v.rhs_off(e) + (size_t)c * nh + i] = rv;
+      for (int k = 0; k < v.nshift; k++) {
+        v.x[v.xs_off(e, k) + (size_t)c * nh + i] = z;
+        v.p[v.xs_off(e, k) + (size_t)c * nh + i] = rv;
       }
     }
   }
-  double tot[kMaxRhs];
-  if (!(grid_reduce<kMaxRhs>(s, partials, ticket, tot) && threadIdx.x == 0)) return;
-  int any = 0;
-  st->itn = 0;
-  for (int j = 0; j < st->nrhs; j++) {
-    st->b2[j] = tot[j];
-    st->r2i[j] = tot[j];
-    st->r2stop[j] = r2req * tot[j];
-    st->alphaim1[j] = -1.0;
-    st->betaim1[j] = 0.0;
-    const int c = (tot[j] > st->r2stop[j]) && isfinite(tot[j]) ? 1 : 0;
-    st->cont[j] = st->live[j] = c;
-    any |= c;
-    for (int k = 0; k < st->nshift; k++) {
+  block_sum<n>(s, sh);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < n; q++)
+      if (e * n + q < nrhs) partials[(size_t)(e * n + q) * gridDim.x + blockIdx.x] = s[q];
+  }
+  double tot;
+  if (!rhs_reduce(nrhs, partials, gridDim.x, ticket, gridDim.x * gridDim.y, tot)) return;
+  const int j = threadIdx.x >> 5, k = threadIdx.x & 31;
+  int c = 0;
+  if (j < nrhs) {
+    c = (tot > r2req * tot) && isfinite(tot) ? 1 : 0;
+    if (k == 0) {
+      st->b2[j] = tot;
+      st->r2i[j] = tot;
+      st->r2stop[j] = r2req * tot;
+      st->alphaim1[j] = -1.0;
+      st->betaim1[j] = 0.0;
+      st->live[j] = c;
+    }
+    if (k < st->nshift) {
       st->zi[j][k] = st->zim1[j][k] = 1.0;
       st->active[j][k] = 1;
       st->dox[j][k] = st->dop[j][k] = 0;
     }
   }
-  st->done = (any && st->maxits > 0) ? 0 : 1;
+  const int any = __syncthreads_or(c);
+  if (threadIdx.x == 0) {
+    st->itn = 0;
+    st->last = 0;
+    st->done = (any && st->maxits > 0) ? 0 : 1;
+  }
 }
 
-// FP32 or FP64 vector -> FP64 block of a full-lattice field
+// right-hand side q of a vector's elements -> FP64 block of a full-lattice field
 template <class VT>
-__global__ void cgm_out_kernel(const VT *x, int nh, double2 *y, int ystride, double scale) {
+__global__ void cgm_out_kernel(const VT *x, int q, int nh, double2 *y, int ystride, double scale) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x)
     for (int c = 0; c < 3; c++) {
       VT v = x[(size_t)c * nh + i];
-      y[(size_t)c * ystride + i] = make_double2(scale * (double)v.x, scale * (double)v.y);
+      y[(size_t)c * ystride + i] = make_double2(scale * (double)lane(v, q).x, scale * (double)lane(v, q).y);
     }
 }
 
@@ -484,13 +620,15 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
   const Geom &geo = g->l->g;
   const int nh = geo.nh;
   Workspace &ws = g->ws;
-  const size_t es = fp32 ? sizeof(float2) : sizeof(double2);
+  const bool pairs = fp32 && nrhs > 1;
+  const int nvec = pairs ? (nrhs + 1) / 2 : nrhs;
+  const size_t es = pairs ? sizeof(float4) : fp32 ? sizeof(float2) : sizeof(double2);
   const size_t vb = es * 3 * (size_t)nh;
   void *pr, *pap, *pt, *px, *pp, *pst, *pb;
   int rc;
-  if ((rc = ws.get(kSlotMs0 + 40, vb * nrhs, &pr)) || (rc = ws.get(kSlotMs0 + 41, vb * nrhs, &pap)) ||
-      (rc = ws.get(kSlotMs0 + 42, vb * nrhs, &pt)) || (rc = ws.get(kSlotMs0 + 43, vb * nrhs * nshift, &px)) ||
-      (rc = ws.get(kSlotMs0 + 44, vb * nrhs * nshift, &pp)) ||
+  if ((rc = ws.get(kSlotMs0 + 40, vb * nvec, &pr)) || (rc = ws.get(kSlotMs0 + 41, vb * nvec, &pap)) ||
+      (rc = ws.get(kSlotMs0 + 42, vb * nvec, &pt)) || (rc = ws.get(kSlotMs0 + 43, vb * nvec * nshift, &px)) ||
+      (rc = ws.get(kSlotMs0 + 44, vb * nvec * nshift, &pp)) ||
       (rc = ws.get(kSlotMs0 + 45, sizeof(CgmState), &pst)) ||
       (rc = ws.get(kSlotMs0 + 46, sizeof(double2 *) * kMaxRhs, &pb)))
     return rc;
@@ -510,66 +648,57 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
   QS_CUDA(cudaMemcpyAsync(st, pin, sizeof(hs), cudaMemcpyHostToDevice, stream()));
   QS_CUDA(cudaMemcpyAsync(pb, (char *)pin + sizeof(hs), sizeof(double2 *) * nrhs, cudaMemcpyHostToDevice,
                           stream()));
-  const int grid = std::min(grid_for(nh, kBlock, 4), kMaxRedBlocks * 8 / kMaxRhs);
-  const int egrid = grid_for(nh, kBlock, 8);
+  // grid rows share the GPU; kMaxRedBlocks slots per right-hand side
+  const dim3 grid(std::min(grid_for(nh, kBlock, std::max(1, 8 / nvec)), kMaxRedBlocks), nvec);
   const int every = check_interval(nh);
-  if (fp32) {
-    CgmVecs<float2> v{(float2 *)pr, (float2 *)pap, (float2 *)pt, (float2 *)px, (float2 *)pp, nh, nshift, nrhs};
-    cgm_init_kernel<float2><<<grid, kBlock, 0, stream()>>>(v, (const double2 *const *)pb, bstride, st,
-                                                           red_partials(), red_tickets(), r2req);
+  // one iteration's kernels after the operator's two half sweeps
+  auto solve = [&](auto v, auto schur) -> int {
+    using VT = std::remove_pointer_t<decltype(v.r)>;
+    cgm_init_kernel<VT><<<grid, kBlock, 0, stream()>>>(v, (const double2 *const *)pb, bstride, st, red_partials(),
+                                                       red_tickets(), r2req);
     note_launch();
     QS_LAUNCH_CHECK();
+    int it = 0;
     for (;;) {
       for (int i = 0; i < every; i++) {
-        // p_0 of right-hand side j lives at xs_off(j, 0)
-        if (nrhs == 1)
-          rc = schur_lo_v32(g, lprec, par, v.ap, v.p, v.t, m2, &st->pAp[0]);
-        else
-          rc = schur_mrhs(g, par, nrhs, v.p, v.xs_off(1, 0), v.t, v.ap, m2, st);
-        if (rc) return rc;
-        cgm_alpha_kernel<<<1, 1, 0, stream()>>>(st);
-        cgm_update1_kernel<float2><<<grid, kBlock, 0, stream()>>>(v, st, red_partials(), red_tickets());
-        cgm_update2_kernel<float2><<<egrid, kBlock, 0, stream()>>>(v, st);
-        cgm_finish_kernel<<<1, 1, 0, stream()>>>(st);
-        note_launch(4);
+        int rc2 = schur(v);
+        if (rc2) return rc2;
+        it++;
+        launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, v, st, red_partials(), red_tickets());
+        launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, v, (const CgmState *)st, it);
+        note_launch(2);
       }
       QS_LAUNCH_CHECK();
-      if ((rc = read_cgm_head(st, &hs))) return rc;
+      int rc2 = read_cgm_head(st, &hs);
+      if (rc2) return rc2;
       if (hs.done) break;
     }
+    constexpr int n = Lanes<VT>::n;
+    const int egrid = grid_for(nh, kBlock, 8);
     for (int j = 0; j < nrhs; j++)
       for (int k = 0; k < nshift; k++) {
-        cgm_out_kernel<float2><<<egrid, kBlock, 0, stream()>>>(v.x + v.xs_off(j, k), nh, y[j * nshift + k],
-                                                               ystride, yscale);
+        cgm_out_kernel<VT><<<egrid, kBlock, 0, stream()>>>(v.x + v.xs_off(j / n, k), j % n, nh, y[j * nshift + k],
+                                                           ystride, yscale);
         note_launch();
       }
+    return QEXSTAG_OK;
+  };
+  if (pairs) {
+    CgmVecs<float4> v{(float4 *)pr, (float4 *)pap, (float4 *)pt, (float4 *)px, (float4 *)pp, nh, nshift, nvec};
+    // p_0 of pair j lives at xs_off(j, 0)
+    rc = solve(v, [&](auto &w) { return schur_mrhs(g, par, nrhs, w.p, w.xs_off(1, 0), w.t, w.ap, m2, st); });
+  } else if (fp32) {
+    CgmVecs<float2> v{(float2 *)pr, (float2 *)pap, (float2 *)pt, (float2 *)px, (float2 *)pp, nh, nshift, 1};
+    rc = solve(v, [&](auto &w) { return schur_lo_v32(g, lprec, par, w.ap, w.p, w.t, m2, &st->pAp[0]); });
   } else {
     if (nrhs != 1) return fail(QEXSTAG_ERR_ARG, "FP64 multi-shift takes one right-hand side");
     CgmVecs<double2> v{(double2 *)pr, (double2 *)pap, (double2 *)pt, (double2 *)px, (double2 *)pp, nh, nshift, 1};
-    cgm_init_kernel<double2><<<grid, kBlock, 0, stream()>>>(v, (const double2 *const *)pb, bstride, st,
-                                                            red_partials(), red_tickets(), r2req);
-    note_launch();
-    QS_LAUNCH_CHECK();
-    for (;;) {
-      for (int i = 0; i < every; i++) {
-        if ((rc = schur64(g, par, VecD{v.ap, nh}, CVecD{v.p, nh}, VecD{v.t, nh}, m2, kRedDot, nullptr,
-                          &st->done, &st->pAp[0])))
-          return rc;
-        cgm_alpha_kernel<<<1, 1, 0, stream()>>>(st);
-        cgm_update1_kernel<double2><<<grid, kBlock, 0, stream()>>>(v, st, red_partials(), red_tickets());
-        cgm_update2_kernel<double2><<<egrid, kBlock, 0, stream()>>>(v, st);
-        cgm_finish_kernel<<<1, 1, 0, stream()>>>(st);
-        note_launch(4);
-      }
-      QS_LAUNCH_CHECK();
-      if ((rc = read_cgm_head(st, &hs))) return rc;
-      if (hs.done) break;
-    }
-    for (int k = 0; k < nshift; k++) {
-      cgm_out_kernel<double2><<<egrid, kBlock, 0, stream()>>>(v.x + v.xs_off(0, k), nh, y[k], ystride, yscale);
-      note_launch();
-    }
+    rc = solve(v, [&](auto &w) {
+      return schur64(g, par, VecD{w.ap, nh}, CVecD{w.p, nh}, VecD{w.t, nh}, m2, kRedDot, nullptr, &st->done,
+                     &st->pAp[0]);
+    });
   }
+  if (rc) return rc;
   QS_LAUNCH_CHECK();
   *iters = hs.itn;
   return QEXSTAG_OK;

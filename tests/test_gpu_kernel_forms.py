@@ -53,3 +53,24 @@ def test_smearing_sweep_remainders(cuda, coef):
     d = d0.copy()
     sm.fat7Deriv(d, g, ch, c)
     assert rel(d, d0 + O.fat7_deriv(dims, coef, g, ch)[0]) < 1e-12
+
+
+# multi-shift solves: 1 (one vector), 2 and 3 (one and two pairs, an odd one
+# with a zero partner), 5 and 8 right-hand sides, on 720 = 22 1/2 sets of sites
+@pytest.mark.parametrize("nrhs,naik", [(1, 1), (2, 1), (3, 1), (3, 0), (5, 1), (8, 0)])
+def test_shifted_systems_by_right_hand_sides(cuda, nrhs, naik):
+    dims, m, sigmas = (4, 6, 6, 10), 0.2, [0.3, 0.0, 1.0]
+    g = F.fat_naik_links(dims, 3) if naik else F.naive_links(dims, 0.3, 3)
+    V = F.volume(dims)
+    o, s = O.Oracle(dims, g), S.Staggered(S.Layout(dims), S.to_device_links(g))
+    bs = [F.even_source(dims, 40 + j) for j in range(nrhs)]
+    ys = [[S.to_device_vector(np.zeros_like(b)) for _ in sigmas] for b in bs]
+    sp = S.SolverParams(r2req=1e-20, sloppySolve=S.L.SLOPPY_SINGLE)
+    r2 = s.cgm_ee(m, sigmas, [S.to_device_vector(b) for b in bs], ys, sp)
+    assert sp.status == S.L.OK and (r2 <= 1e-20).all()
+    for b, row in zip(bs, ys):
+        for sg, y in zip(sigmas, row):
+            y, ay = S.to_host_vector(y), o.vec()
+            o.stagD2ee(ay, y, m * m + 0.25 * sg)
+            assert np.linalg.norm((ay - b)[: V // 2]) <= 1.01e-10 * np.linalg.norm(b)
+            assert not np.any(y[V // 2:])
