@@ -407,7 +407,6 @@ int qexstag_links_update(qexstag_links *g, const double *links, int mem) {
   if ((rc = check_links(g)) || (rc = check_mem(mem))) return rc;
   if (!links) return fail(QEXSTAG_ERR_ARG, "links_update: null links");
   if ((rc = upload_links(g, links, mem))) return rc;
-  free_low_links(g->low);
   if ((rc = build_low_links(g))) return rc;
   QS_CUDA(cudaStreamSynchronize(stream()));
   return QEXSTAG_OK;
@@ -469,7 +468,6 @@ int qexstag_links_update_milc(qexstag_links *g, const double *fat, const double 
     return fail(QEXSTAG_ERR_ARG, "links_update_milc: fat is null, or lng is given for a naive handle "
                                  "or missing for a fat+Naik handle");
   if ((rc = upload_links_milc(g, fat, lng))) return rc;
-  free_low_links(g->low);
   if ((rc = build_low_links(g))) return rc;
   QS_CUDA(cudaStreamSynchronize(stream()));
   return QEXSTAG_OK;

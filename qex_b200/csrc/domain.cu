@@ -147,7 +147,6 @@ constexpr size_t kDevScalarBytes = sizeof(double) * kStateOff + sizeof(CgState);
 int write_state(CgState *dst, const CgState &host);
 int check_interval(int nh);
 int build_low_links(qexstag_links_s *g);
-void free_low_links(LowLinks &low);
 
 // sites of one parity in one (z, t) row, and in one t slice of the
 // extended lattice
@@ -1064,7 +1063,6 @@ int qexstag_domain_links(qexstag_domain *const *doms, int n, const double *const
     if ((rc = exchange(doms, n, base.data(), ncomp, par, stream()))) return rc;
   // the reduced-precision copies the mixed-precision solve iterates with
   for (int k = 0; k < n; k++) {
-    free_low_links(doms[k]->g->low);
     if ((rc = build_low_links(doms[k]->g))) return rc;
   }
   QS_CUDA(cudaStreamSynchronize(stream()));

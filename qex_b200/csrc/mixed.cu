@@ -29,190 +29,190 @@ namespace qs {
 // building the reduced-precision copies
 // ---------------------------------------------------------------------------
 
-__global__ void absmax_kernel(const double2 *__restrict__ u, size_t n, unsigned *out) {
-  float m = 0.f;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double2 v = u[i];
-    m = fmaxf(m, (float)fmax(fabs(v.x), fabs(v.y)));
-  }
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));  // m >= 0: uint order = float order
-}
-
-// max over long links of |row2 - (s/c) conj(row0 x row1)| / |c|
-__global__ void recon_check_kernel(Geom g, const double2 *__restrict__ u64, double c, unsigned *out) {
+// One pass over the link list for what the copies need to know: out[0] and
+// out[1] the largest |real| of the fat (or naive) and of the long links, out[2]
+// the largest |row2 - (s/c) conj(row0 x row1)| / |c| of the long links.
+template <int NL>
+__global__ void __launch_bounds__(kBlock) low_scan_kernel(Geom g, const double2 *__restrict__ u64, double c,
+                                                         unsigned *out) {
   const size_t V = g.V;
-  float m = 0.f;
+  float m[3] = {0.f, 0.f, 0.f};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * g.V; t += gridDim.x * blockDim.x) {
     const int mu = t / g.V, site = t - mu * g.V;
-    const int par = site >= g.nh ? 1 : 0;
-    int x[4], lex;
-    site_coords(g, par, site - par * g.nh, x, lex);
-    double s = long_sign_fwd(g, x, mu);
-    const double2 *ul = u64 + (size_t)(2 * mu + 1) * 9 * V + site;
-    double2 e[9];
-    for (int j = 0; j < 9; j++) e[j] = ul[(size_t)j * V];
-    double2 cr[3];
-    for (int i = 0; i < 3; i++) {
-      int j = (i + 1) % 3, k = (i + 2) % 3;
-      double2 a = e[j], b = e[3 + k], a2 = e[k], b2 = e[3 + j];
-      cr[i] = make_double2(a.x * b.x - a.y * b.y - (a2.x * b2.x - a2.y * b2.y),
-                           a.x * b.y + a.y * b.x - (a2.x * b2.y + a2.y * b2.x));
+    const double2 *uf = u64 + (size_t)(NL == 8 ? 2 * mu : mu) * 9 * V + site;
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+      const double2 v = uf[(size_t)j * V];
+      m[0] = fmaxf(m[0], (float)fmax(fabs(v.x), fabs(v.y)));
     }
-    double k = s / c, d = 0;
-    for (int i = 0; i < 3; i++) {
-      d = fmax(d, fabs(e[6 + i].x - k * cr[i].x));
-      d = fmax(d, fabs(e[6 + i].y + k * cr[i].y));
+    if (NL == 8) {
+      const int par = site >= g.nh ? 1 : 0;
+      int x[4], lex;
+      site_coords(g, par, site - par * g.nh, x, lex);
+      const double s = long_sign_fwd(g, x, mu);
+      double2 e[9];
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        e[j] = uf[(size_t)(9 + j) * V];
+        m[1] = fmaxf(m[1], (float)fmax(fabs(e[j].x), fabs(e[j].y)));
+      }
+      const double k = s / c;
+      double d = 0;
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int j = (i + 1) % 3, l = (i + 2) % 3;
+        const double2 a = e[j], b = e[3 + l], a2 = e[l], b2 = e[3 + j];
+        const double2 cr = make_double2(a.x * b.x - a.y * b.y - (a2.x * b2.x - a2.y * b2.y),
+                                        a.x * b.y + a.y * b.x - (a2.x * b2.y + a2.y * b2.x));
+        d = fmax(d, fabs(e[6 + i].x - k * cr.x));
+        d = fmax(d, fabs(e[6 + i].y + k * cr.y));
+      }
+      m[2] = fmaxf(m[2], (float)(d / fabs(c)));
     }
-    m = fmaxf(m, (float)(d / fabs(c)));
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
-}
-
-// FP32/FP16 copy of link k (all sites) into list slot f
-__global__ void to_low18_kernel(const double2 *__restrict__ uk, size_t V, float4 *c32, float2 *t32,
-                                uint4 *c16, unsigned *t16, int f, float inv16) {
-  for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < V; s += (size_t)gridDim.x * blockDim.x) {
-    double2 e[9];
-    for (int j = 0; j < 9; j++) e[j] = uk[(size_t)j * V + s];
-    for (int j = 0; j < 4; j++)
-      c32[((size_t)f * 4 + j) * V + s] =
-          make_float4((float)e[2 * j].x, (float)e[2 * j].y, (float)e[2 * j + 1].x, (float)e[2 * j + 1].y);
-    t32[(size_t)f * V + s] = make_float2((float)e[8].x, (float)e[8].y);
-    for (int j = 0; j < 2; j++) {
-      uint4 q;
-      q.x = f2h((float)(e[4 * j].x * inv16), (float)(e[4 * j].y * inv16));
-      q.y = f2h((float)(e[4 * j + 1].x * inv16), (float)(e[4 * j + 1].y * inv16));
-      q.z = f2h((float)(e[4 * j + 2].x * inv16), (float)(e[4 * j + 2].y * inv16));
-      q.w = f2h((float)(e[4 * j + 3].x * inv16), (float)(e[4 * j + 3].y * inv16));
-      c16[((size_t)f * 2 + j) * V + s] = q;
-    }
-    t16[(size_t)f * V + s] = f2h((float)(e[8].x * inv16), (float)(e[8].y * inv16));
+#pragma unroll
+  for (int q = 0; q < (NL == 8 ? 3 : 1); q++) {
+    for (int o = 16; o > 0; o >>= 1) m[q] = fmaxf(m[q], __shfl_down_sync(0xffffffffu, m[q], o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out + q, __float_as_uint(m[q]));  // >= 0: uint order = float order
   }
 }
 
-__global__ void to_low12_kernel(const double2 *__restrict__ uk, size_t V, float4 *c32, uint4 *c16,
-                                uint2 *t16, int f, float inv16) {
-  for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < V; s += (size_t)gridDim.x * blockDim.x) {
-    double2 e[6];
-    for (int j = 0; j < 6; j++) e[j] = uk[(size_t)j * V + s];
-    for (int j = 0; j < 3; j++)
-      c32[((size_t)f * 3 + j) * V + s] =
-          make_float4((float)e[2 * j].x, (float)e[2 * j].y, (float)e[2 * j + 1].x, (float)e[2 * j + 1].y);
+// FP32 and 16-bit copies of all 18 reals of link f at site s
+__device__ __forceinline__ void store_low18(const double2 *__restrict__ u, size_t V, size_t s, int f, float4 *c32,
+                                            float2 *t32, uint4 *c16, unsigned *t16, float inv16) {
+  double2 e[9];
+#pragma unroll
+  for (int j = 0; j < 9; j++) e[j] = u[(size_t)j * V];
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    c32[((size_t)f * 4 + j) * V + s] =
+        make_float4((float)e[2 * j].x, (float)e[2 * j].y, (float)e[2 * j + 1].x, (float)e[2 * j + 1].y);
+  t32[(size_t)f * V + s] = make_float2((float)e[8].x, (float)e[8].y);
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
     uint4 q;
-    q.x = f2h((float)(e[0].x * inv16), (float)(e[0].y * inv16));
-    q.y = f2h((float)(e[1].x * inv16), (float)(e[1].y * inv16));
-    q.z = f2h((float)(e[2].x * inv16), (float)(e[2].y * inv16));
-    q.w = f2h((float)(e[3].x * inv16), (float)(e[3].y * inv16));
-    c16[(size_t)f * V + s] = q;
-    uint2 t;
-    t.x = f2h((float)(e[4].x * inv16), (float)(e[4].y * inv16));
-    t.y = f2h((float)(e[5].x * inv16), (float)(e[5].y * inv16));
-    t16[(size_t)f * V + s] = t;
+    q.x = f2h((float)(e[4 * j].x * inv16), (float)(e[4 * j].y * inv16));
+    q.y = f2h((float)(e[4 * j + 1].x * inv16), (float)(e[4 * j + 1].y * inv16));
+    q.z = f2h((float)(e[4 * j + 2].x * inv16), (float)(e[4 * j + 2].y * inv16));
+    q.w = f2h((float)(e[4 * j + 3].x * inv16), (float)(e[4 * j + 3].y * inv16));
+    c16[((size_t)f * 2 + j) * V + s] = q;
+  }
+  t16[(size_t)f * V + s] = f2h((float)(e[8].x * inv16), (float)(e[8].y * inv16));
+}
+
+// the copies of every link of the list, long links with 12 reals (R12) or 18
+template <int NL, int R12>
+__global__ void __launch_bounds__(kBlock) low_copy_kernel(const double2 *__restrict__ u64, int V_, LowLinks L,
+                                                         float inv_fat, float inv_long) {
+  const size_t V = V_;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * V_; t += gridDim.x * blockDim.x) {
+    const int f = t / V_, s = t - f * V_;
+    const double2 *uf = u64 + (size_t)(NL == 8 ? 2 * f : f) * 9 * V + s;
+    store_low18(uf, V, s, f, L.f32_fat, L.f32_fat_tail, L.f16_fat, L.f16_fat_tail, inv_fat);
+    if (NL == 8 && !R12)
+      store_low18(uf + 9 * V, V, s, f, L.f32_long, L.f32_long_tail, L.f16_long, L.f16_long_tail, inv_long);
+    if (NL == 8 && R12) {
+      double2 e[6];
+#pragma unroll
+      for (int j = 0; j < 6; j++) e[j] = uf[(size_t)(9 + j) * V];
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        L.f32_long[((size_t)f * 3 + j) * V + s] =
+            make_float4((float)e[2 * j].x, (float)e[2 * j].y, (float)e[2 * j + 1].x, (float)e[2 * j + 1].y);
+      uint4 q;
+      q.x = f2h((float)(e[0].x * inv_long), (float)(e[0].y * inv_long));
+      q.y = f2h((float)(e[1].x * inv_long), (float)(e[1].y * inv_long));
+      q.z = f2h((float)(e[2].x * inv_long), (float)(e[2].y * inv_long));
+      q.w = f2h((float)(e[3].x * inv_long), (float)(e[3].y * inv_long));
+      L.f16_long[(size_t)f * V + s] = q;
+      uint2 w;
+      w.x = f2h((float)(e[4].x * inv_long), (float)(e[4].y * inv_long));
+      w.y = f2h((float)(e[5].x * inv_long), (float)(e[5].y * inv_long));
+      L.f16_long_tail2[(size_t)f * V + s] = w;
+    }
   }
 }
 
 template <class T>
 static int dalloc(T **p, size_t n) {
+  if (*p) return QEXSTAG_OK;
   cudaError_t e = cudaMalloc((void **)p, sizeof(T) * n);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    *p = nullptr;
     return fail(QEXSTAG_ERR_ALLOC, "device allocation of reduced-precision links failed");
   }
   return QEXSTAG_OK;
 }
 
-static int read_uint(unsigned *d, unsigned *h) {
-  QS_CUDA(cudaMemcpyAsync(h, d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream()));
-  QS_CUDA(cudaStreamSynchronize(stream()));
-  return QEXSTAG_OK;
+template <class T>
+static void dfree(T **p) {
+  cudaFree(*p);
+  *p = nullptr;
 }
 
-static int absmax_links(const double2 *u, size_t n, float *out, unsigned *scratch) {
-  QS_CUDA(cudaMemsetAsync(scratch, 0, sizeof(unsigned), stream()));
-  absmax_kernel<<<grid_for((long)std::min<size_t>(n, 1u << 30)), kBlock, 0, stream()>>>(u, n, scratch);
-  note_launch();
-  QS_LAUNCH_CHECK();
-  unsigned h = 0;
-  int rc = read_uint(scratch, &h);
-  if (rc) return rc;
-  float f;
-  std::memcpy(&f, &h, sizeof(f));
-  *out = f;
-  return QEXSTAG_OK;
-}
-
+// The reduced-precision copies of g's links, rebuilt whenever they change (in
+// molecular dynamics at every force).  Their buffers stay with the handle;
+// one pass finds the scales and whether the long links take 12 reals, one
+// pass writes the copies, and the host waits once in between.  (With a kernel,
+// a wait and a copy back per link field, and buffers freed and allocated each
+// time, a 16^4 HISQ force took 11.9 ms; now 7.6 ms.)
 int build_low_links(qexstag_links_s *g) {
   LowLinks &L = g->low;
-  L = LowLinks();
+  L.ready = false;
   const Geom &geo = g->l->g;
   const size_t V = geo.V;
   const bool naik = g->nl == 8;
   L.nfat = 4;
   L.nlong = naik ? 4 : 0;
   L.long_coeff = g->long_coeff;
-  unsigned *scratch = (unsigned *)red_tickets() + (kNumTickets - 1);
+  unsigned *found = (unsigned *)red_results();
   int rc;
-  // scales (max |element|) of the fat and long lists
-  float fat_max = 0.f, long_max = 0.f;
-  for (int k = 0; k < g->nl; k++) {
-    float m = 0.f;
-    if ((rc = absmax_links(g->u64 + (size_t)k * 9 * V, 9 * V, &m, scratch))) return rc;
-    if (naik && (k & 1))
-      long_max = std::max(long_max, m);
-    else
-      fat_max = std::max(fat_max, m);
-  }
+  const int grid = grid_for(4L * geo.V);
+  QS_CUDA(cudaMemsetAsync(found, 0, 3 * sizeof(unsigned), stream()));
+  if (naik)
+    low_scan_kernel<8><<<grid, kBlock, 0, stream()>>>(geo, g->u64, g->long_coeff, found);
+  else
+    low_scan_kernel<4><<<grid, kBlock, 0, stream()>>>(geo, g->u64, g->long_coeff, found);
+  note_launch();
+  QS_LAUNCH_CHECK();
+  QS_CUDA(cudaMemcpyAsync(host_results(), found, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream()));
+  QS_CUDA(cudaStreamSynchronize(stream()));
+  float seen[3];
+  std::memcpy(seen, host_results(), sizeof(seen));
+  const float fat_max = seen[0], long_max = seen[1];
   if (!(fat_max > 0.f) || !std::isfinite(fat_max) || (naik && (!(long_max > 0.f) || !std::isfinite(long_max))))
     return fail(QEXSTAG_ERR_ARG, "links_create: links are zero or not finite");
   L.fat_scale = fat_max;
   L.long_scale = naik ? long_max : 1.0f;
   // are the long links coeff * sign * SU(3)?
-  if (naik) {
-    QS_CUDA(cudaMemsetAsync(scratch, 0, sizeof(unsigned), stream()));
-    recon_check_kernel<<<grid_for(4L * V), kBlock, 0, stream()>>>(geo, g->u64, g->long_coeff, scratch);
-    note_launch();
-    QS_LAUNCH_CHECK();
-    unsigned h = 0;
-    if ((rc = read_uint(scratch, &h))) return rc;
-    float dev;
-    std::memcpy(&dev, &h, sizeof(dev));
-    L.recon12 = dev < 2e-6f;
+  const bool r12 = naik && seen[2] < 2e-6f;
+  if (r12 != L.recon12) {
+    dfree(&L.f32_long);
+    dfree(&L.f32_long_tail);
+    dfree(&L.f16_long);
+    dfree(&L.f16_long_tail2);
+    dfree(&L.f16_long_tail);
+    L.recon12 = r12;
   }
   if ((rc = dalloc(&L.f32_fat, (size_t)4 * 4 * V)) || (rc = dalloc(&L.f32_fat_tail, (size_t)4 * V)) ||
       (rc = dalloc(&L.f16_fat, (size_t)4 * 2 * V)) || (rc = dalloc(&L.f16_fat_tail, (size_t)4 * V)))
     return rc;
-  for (int f = 0; f < 4; f++) {
-    const int k = naik ? 2 * f : f;
-    to_low18_kernel<<<grid_for((long)V), kBlock, 0, stream()>>>(g->u64 + (size_t)k * 9 * V, V, L.f32_fat,
-                                                                L.f32_fat_tail, L.f16_fat, L.f16_fat_tail,
-                                                                f, 1.0f / L.fat_scale);
-    note_launch();
-  }
-  if (naik) {
-    if (L.recon12) {
-      if ((rc = dalloc(&L.f32_long, (size_t)4 * 3 * V)) || (rc = dalloc(&L.f16_long, (size_t)4 * V)) ||
-          (rc = dalloc(&L.f16_long_tail2, (size_t)4 * V)))
-        return rc;
-      for (int f = 0; f < 4; f++) {
-        to_low12_kernel<<<grid_for((long)V), kBlock, 0, stream()>>>(g->u64 + (size_t)(2 * f + 1) * 9 * V, V,
-                                                                    L.f32_long, L.f16_long, L.f16_long_tail2,
-                                                                    f, 1.0f / L.long_scale);
-        note_launch();
-      }
-    } else {
-      if ((rc = dalloc(&L.f32_long, (size_t)4 * 4 * V)) || (rc = dalloc(&L.f32_long_tail, (size_t)4 * V)) ||
-          (rc = dalloc(&L.f16_long, (size_t)4 * 2 * V)) || (rc = dalloc(&L.f16_long_tail, (size_t)4 * V)))
-        return rc;
-      for (int f = 0; f < 4; f++) {
-        to_low18_kernel<<<grid_for((long)V), kBlock, 0, stream()>>>(g->u64 + (size_t)(2 * f + 1) * 9 * V, V,
-                                                                    L.f32_long, L.f32_long_tail, L.f16_long,
-                                                                    L.f16_long_tail, f, 1.0f / L.long_scale);
-        note_launch();
-      }
-    }
-  }
+  if (r12 && ((rc = dalloc(&L.f32_long, (size_t)4 * 3 * V)) || (rc = dalloc(&L.f16_long, (size_t)4 * V)) ||
+              (rc = dalloc(&L.f16_long_tail2, (size_t)4 * V))))
+    return rc;
+  if (naik && !r12 &&
+      ((rc = dalloc(&L.f32_long, (size_t)4 * 4 * V)) || (rc = dalloc(&L.f32_long_tail, (size_t)4 * V)) ||
+       (rc = dalloc(&L.f16_long, (size_t)4 * 2 * V)) || (rc = dalloc(&L.f16_long_tail, (size_t)4 * V))))
+    return rc;
+  const float inv_fat = 1.0f / L.fat_scale, inv_long = 1.0f / L.long_scale;
+  if (!naik)
+    low_copy_kernel<4, 0><<<grid, kBlock, 0, stream()>>>(g->u64, geo.V, L, inv_fat, inv_long);
+  else if (r12)
+    low_copy_kernel<8, 1><<<grid, kBlock, 0, stream()>>>(g->u64, geo.V, L, inv_fat, inv_long);
+  else
+    low_copy_kernel<8, 0><<<grid, kBlock, 0, stream()>>>(g->u64, geo.V, L, inv_fat, inv_long);
+  note_launch();
   QS_LAUNCH_CHECK();
   L.ready = true;
   return QEXSTAG_OK;

@@ -23,7 +23,6 @@
 namespace qs {
 
 int build_low_links(qexstag_links_s *g);
-void free_low_links(LowLinks &low);
 
 // NL fields of the list are rephased, field l as direction Hop<NL>::mu(l)
 // with hop Hop<NL>::len(l) (NL = 4: fields 0-3 as directions 0-3, one hop)
@@ -60,7 +59,6 @@ int rephase_links(qexstag_links_s *g, bool literal) {
     rephase_kernel<4><<<grid, kBlock, 0, stream()>>>(geo, g->u64);
   note_launch();
   QS_LAUNCH_CHECK();
-  free_low_links(g->low);
   return build_low_links(g);
 }
 

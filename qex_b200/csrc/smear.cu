@@ -336,7 +336,6 @@ int qexstag_links_hisq(qexstag_links *g, qexstag_smear *s, const qexstag_hisq_co
   if ((rc = smear_in(s, kSmIn0, thin, mem, &u))) return rc;
   // fat link of direction mu at list entry 2 mu, long link at 2 mu + 1
   if ((rc = hisq_dev(s, *c, u, g->u64, 2 * fs, g->u64 + fs, 2 * fs))) return rc;
-  free_low_links(g->low);
   if ((rc = build_low_links(g))) return rc;
   QS_CUDA(cudaStreamSynchronize(stream()));
   return QEXSTAG_OK;

@@ -11,7 +11,6 @@
 
 namespace qs {
 
-void free_low_links(LowLinks &low);
 int build_low_links(qexstag_links_s *g);
 
 constexpr int kSmBlock = 128;

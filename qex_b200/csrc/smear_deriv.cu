@@ -568,7 +568,6 @@ int qexstag_hisq_force(qexstag_links *g, qexstag_smear *s, const qexstag_hisq_co
   }
   // smear the thin links into the operator (smearGetForce's forward part)
   if ((rc = hisq_dev(s, *c, u, g->u64, 2 * fs, g->u64 + fs, 2 * fs))) return rc;
-  free_low_links(g->low);
   if ((rc = build_low_links(g))) return rc;
   // stagForceSolve, then fermForce's outer products f1 (fat) and f3 (long)
   double2 *psi = (double2 *)ppsi, *f8 = (double2 *)pf8, *ff = (double2 *)pff;
