@@ -67,6 +67,19 @@ int Workspace::get_pinned(size_t bytes, void **out) {
   return QEXSTAG_OK;
 }
 
+int Workspace::get_progress(unsigned long long **out) {
+  if (!progress) {
+    cudaError_t e = cudaHostAlloc((void **)&progress, sizeof(*progress), cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      progress = nullptr;
+      return fail(QEXSTAG_ERR_ALLOC, "pinned host allocation failed");
+    }
+  }
+  *out = progress;
+  return QEXSTAG_OK;
+}
+
 void Workspace::release() {
   cudaStreamSynchronize(stream());
   for (auto &kv : bufs) cudaFree(kv.second.second);
@@ -74,6 +87,8 @@ void Workspace::release() {
   if (pinned) cudaFreeHost(pinned);
   pinned = nullptr;
   pinned_bytes = 0;
+  if (progress) cudaFreeHost(progress);
+  progress = nullptr;
 }
 
 // ---- staging of full-lattice colour vectors ----

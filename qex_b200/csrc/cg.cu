@@ -130,6 +130,35 @@ int StateSnapshot::wait(void *host, size_t bytes) {
   return QEXSTAG_OK;
 }
 
+int Pace::start(Workspace &ws, int nh) {
+  int rc = ws.get_progress(&word);
+  if (rc) return rc;
+  // a word of no epoch: nothing done yet (kernels of an earlier solve on this
+  // handle are over, or return without posting an epoch that is waited for)
+  *(volatile unsigned long long *)word = 0;
+  queued = base = epoch = 0;
+  // enough queued work to cover a launch's way to the GPU and the report's
+  // way back (tens of us)
+  depth = nh <= (1 << 15) ? 6 : nh <= (1 << 17) ? 4 : 2;
+  return QEXSTAG_OK;
+}
+
+int Pace::wait(unsigned long long *seen) {
+  for (unsigned spins = 0;; spins++) {
+    const unsigned long long v = *(volatile unsigned long long *)word;
+    *seen = v;
+    if (now(v) && (v & (kPaceStop | kPacePending))) return QEXSTAG_OK;
+    if (queued - (now(v) ? (unsigned)v : base) < depth) return QEXSTAG_OK;
+    if ((spins & 0xfff) == 0xfff) {
+      // nothing left to run and still no word: a launch or a kernel failed
+      const cudaError_t e = cudaStreamQuery(stream());
+      if (e == cudaSuccess && *(volatile unsigned long long *)word == v)
+        return fail(QEXSTAG_ERR_STATE, "solve: the queued iterations ended without a report");
+      if (e != cudaSuccess && e != cudaErrorNotReady) return cuda_fail(e, "solve");
+    }
+  }
+}
+
 // iterations enqueued between host checks: small lattices run many
 // iterations per check (launch-bound), large ones few (each is long)
 int check_interval(int nh) {
@@ -162,32 +191,28 @@ int cg64(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, double r2req, 
                                                 st, red_partials(), red_tickets());
   note_launch();
   QS_LAUNCH_CHECK();
-  const int every = check_interval(nh);
   const int pgrid = grid_for(nh, kBlock, 8);
-  auto batch = [&]() -> int {
-    for (int i = 0; i < every; i++) {
-      launch_pdl(cg_p_kernel, pgrid, kBlock, (const double2 *)r.p, r.stride, p.p, p.stride, nh,
-                 (const CgState *)st);
-      note_launch();
-      int rc2 = schur64(g, par, ap, cv(p), t, m2, kRedCgPAp, st, &st->done);
-      if (rc2) return rc2;
-      launch_pdl(cg_xr_kernel, grid, kBlock, x.p, x.stride, r.p, r.stride, (const double2 *)p.p, p.stride,
-                 (const double2 *)ap.p, ap.stride, nh, st, red_partials(), red_tickets());
-      note_launch();
-    }
-    QS_LAUNCH_CHECK();
-    return QEXSTAG_OK;
-  };
-  // The state is read one batch behind: the next batch is queued before
-  // the host waits for the snapshot, so the GPU does not idle during the
-  // check; once the solve is done that batch's kernels return at once.
-  StateSnapshot snap;
-  if ((rc = batch())) return rc;
+  Pace pace;
+  if ((rc = pace.start(ws, nh))) return rc;
+  Progress progress;
+  progress.word = pace.word;
+  progress.itn = &st->itn;
+  progress.stop = &st->done;
   for (;;) {
-    if ((rc = snap.start(st, sizeof(CgState))) || (rc = batch()) || (rc = snap.wait(&hs, sizeof(CgState))))
-      return rc;
-    if (hs.done) break;
+    unsigned long long seen;
+    if ((rc = pace.wait(&seen))) return rc;
+    if (seen & kPaceStop) break;
+    launch_pdl(cg_p_kernel, pgrid, kBlock, (const double2 *)r.p, r.stride, p.p, p.stride, nh, (const CgState *)st);
+    note_launch();
+    if ((rc = schur64(g, par, ap, cv(p), t, m2, kRedCgPAp, st, &st->done, nullptr, progress))) return rc;
+    launch_pdl(cg_xr_kernel, grid, kBlock, x.p, x.stride, r.p, r.stride, (const double2 *)p.p, p.stride,
+               (const double2 *)ap.p, ap.stride, nh, st, red_partials(), red_tickets());
+    note_launch();
+    QS_LAUNCH_CHECK();
+    pace.queued++;
   }
+  StateSnapshot snap;
+  if ((rc = snap.start(st, sizeof(CgState))) || (rc = snap.wait(&hs, sizeof(CgState)))) return rc;
   out->iterations = hs.itn;
   out->r2 = hs.b2 > 0 ? hs.r2 / hs.b2 : 0.0;
   out->nan = hs.nan;

@@ -44,6 +44,7 @@ struct DslashArgs64 {
   // instead nsites / rowlen runs of rowlen sites, pitch apart, from k0
   int k0, n1, k2, nsites;
   int rowlen, pitch;
+  Progress progress;  // posted by this launch (a solve's first half sweep)
 };
 
 // j-th output site of the launch, as an index of the parity block
@@ -75,6 +76,7 @@ __device__ __forceinline__ void reduce_pap(const DslashArgs64 &A, double dot) {
 template <int NL, int HOP, int INIT, int RED>
 __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) {
   pdl_wait();
+  post_progress(A.progress);
   if (A.done != nullptr && *A.done) return;
   const Geom &g = A.g;
   const int nh = g.nh;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
   constexpr int kTerms = 2 * NL, kPer = kTerms / kSplitWarps;
   __shared__ double2 term[kTerms][3][kSplitSites];
   pdl_wait();
+  post_progress(A.progress);
   if (A.done != nullptr && *A.done) return;
   const Geom &g = A.g;
   const int nh = g.nh;
@@ -303,9 +306,10 @@ static int dispatch64(const DslashArgs64 &A, int hop, int init, int red) {
 
 int dslash64(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, CVecD rin,
              double a, double b, double c, int hop, int init, int red, void *state,
-             const int *done, double *dot_out) {
+             const int *done, double *dot_out, const Progress &progress) {
   const Geom &g = gl->l->g;
   DslashArgs64 A;
+  A.progress = progress;
   A.g = g;
   A.po = po;
   A.u = gl->u64;
@@ -344,8 +348,7 @@ int dslash64_ranges(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVec
   const Geom &g = gl->l->g;
   if (k0 < 0 || k1 < k0 || k2 < 0 || k3 < k2 || k1 > g.nh || k3 > g.nh)
     return fail(QEXSTAG_ERR_ARG, "dslash64_ranges: site range outside the parity block");
-  DslashArgs64 A;
-  std::memset(&A, 0, sizeof(A));
+  DslashArgs64 A = {};
   A.g = g;
   A.po = po;
   A.u = gl->u64;
@@ -379,8 +382,7 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
   if (k0 < 0 || nrun < 0 || rowlen < 0 || rowlen > pitch ||
       (nrun > 0 && (long)k0 + (long)(nrun - 1) * pitch + rowlen > g.nh))
     return fail(QEXSTAG_ERR_ARG, "dslash64_rows: site runs outside the parity block");
-  DslashArgs64 A;
-  std::memset(&A, 0, sizeof(A));
+  DslashArgs64 A = {};
   A.g = g;
   A.po = po;
   A.u = gl->u64;
@@ -409,9 +411,9 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
 // stagD2xx (stagD.nim:485-512): t_q = (2D)_{q,par} x (stagDP, rir := 0), then
 // r = 4 m2 x - (2D)_{par,q} t (stagDM with rir := 4 m2 x).
 int schur64(const qexstag_links_s *gl, int par, VecD r, CVecD x, VecD t, double m2, int red,
-            void *state, const int *done, double *dot_out) {
+            void *state, const int *done, double *dot_out, const Progress &progress) {
   int rc = dslash64(gl, 1 - par, t, x, CVecD{nullptr, 0}, CVecD{nullptr, 0}, 0.0, 0.0, 1.0, +1,
-                    0, kRedNone, nullptr, done);
+                    0, kRedNone, nullptr, done, nullptr, progress);
   if (rc) return rc;
   return dslash64(gl, par, r, cv(t), x, CVecD{nullptr, 0}, 0.0, 4.0 * m2, 1.0, -1, 1, red, state,
                   done, dot_out);
@@ -426,8 +428,7 @@ namespace qs {
 // early exit); used by the allocation-free entry point.
 int schur64_plain(const qexstag_links_s *gl, int par, VecD r, CVecD x, VecD t, double m2) {
   const Geom &g = gl->l->g;
-  DslashArgs64 A;
-  std::memset(&A, 0, sizeof(A));
+  DslashArgs64 A = {};
   A.g = g;
   A.u = gl->u64;
   A.n1 = A.nsites = g.nh;

@@ -250,6 +250,29 @@ struct CgState {
   int pad[3];
 };
 
+// A running solve's report to the host, one 64-bit word in pinned memory:
+// iterations done, the flags below and the epoch (reliable updates done) they
+// belong to, from where the solve keeps them on the device.  The first half
+// sweep of an iteration posts it: a kernel is not over before such a write is
+// (about 2 us), and that kernel's own work covers the wait.
+struct Progress {
+  unsigned long long *word = nullptr;
+  const int *itn = nullptr, *stop = nullptr;
+  const int *pending = nullptr, *pin = nullptr, *epoch = nullptr;  // null: 0
+};
+constexpr unsigned long long kPaceStop = 1ull << 32;     // the solve has ended
+constexpr unsigned long long kPacePending = 1ull << 33;  // a reliable update is due
+constexpr unsigned long long kPacePin = 1ull << 34;      // and corrects direction buffer 1, not 0
+__device__ __forceinline__ void post_progress(const Progress &p) {
+  if (p.word == nullptr || blockIdx.x != 0 || threadIdx.x != 0) return;
+  unsigned long long v = (unsigned)*p.itn;
+  if (*p.stop) v |= kPaceStop;
+  if (p.pending && *p.pending) v |= kPacePending;
+  if (p.pin && *p.pin) v |= kPacePin;
+  if (p.epoch) v |= (unsigned long long)(*p.epoch & 0xffffff) << 40;
+  asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p.word), "l"(v) : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // host side: error reporting and per-device runtime
 // ---------------------------------------------------------------------------

@@ -356,11 +356,13 @@ struct DslashArgsLo {
   // output sites [k_lo, min(k_hi, nh)) of the parity (a domain's interior or
   // its intermediate slices); site k is stored at index k - out_off of out
   int k_lo = 0, k_hi = 0x7fffffff, out_off = 0;
+  Progress progress;  // posted by this launch (a solve's first half sweep)
 };
 
 template <int PREC, int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12>
 __global__ void __launch_bounds__(kBlock, PREC == kF16 ? 4 : 1) dslash_lo_kernel(const DslashArgsLo A) {
   pdl_wait();
+  post_progress(A.progress);
   if (A.halt != nullptr && mx_halt(A.halt)) return;
   const Geom &g = A.g;
   const int nh = g.nh;
@@ -483,6 +485,7 @@ __global__ void __launch_bounds__(kBlock, PREC == kF16 ? 4 : 1) dslash_lo_kernel
 template <int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12>
 __global__ void __launch_bounds__(kBlock, 4) dslash_x2_kernel(const DslashArgsLo A) {
   pdl_wait();
+  post_progress(A.progress);
   if (A.halt != nullptr && mx_halt(A.halt)) return;
   const Geom &g = A.g;
   const int nh = g.nh;
@@ -680,7 +683,7 @@ static int sloppy_half(int which, const DslashArgsLo &A, int grid, int red, int 
 // adds the Re <rdot, ap> partials.
 int schur_lo(const qexstag_links_s *g, int prec, int par, float2 *ap, const void *p, void *t,
              double m2, int red, const MxState *halt, double *dot_out, int *red_blocks,
-             const float2 *rdot = nullptr) {
+             const float2 *rdot = nullptr, const Progress &progress = Progress()) {
   const Geom &geo = g->l->g;
   DslashArgsLo A;
   A.g = geo;
@@ -699,6 +702,7 @@ int schur_lo(const qexstag_links_s *g, int prec, int par, float2 *ap, const void
   A.out = t;
   A.ostride = geo.nh;
   A.b = 0.f;
+  A.progress = progress;
   int rc;
   if (prec == kF32)
     rc = g->nl == 8 ? sloppy_half<kF32, 8>(0, A, grid, 0, nullptr) : sloppy_half<kF32, 4>(0, A, grid, 0, nullptr);
@@ -706,6 +710,7 @@ int schur_lo(const qexstag_links_s *g, int prec, int par, float2 *ap, const void
     rc = g->nl == 8 ? sloppy_half<kF16, 8>(0, A, grid, 0, nullptr) : sloppy_half<kF16, 4>(0, A, grid, 0, nullptr);
   if (rc) return rc;
   // half sweep 2
+  A.progress = Progress();
   A.po = par;
   A.xin = t;
   A.xs = p;
@@ -726,7 +731,7 @@ int schur_lo(const qexstag_links_s *g, int prec, int par, float2 *ap, const void
 // single-right-hand-side multi-shift CG): ap = 4 m2 p - (2D)(2D) p on parity
 // par, t the FP32 temporary, *dot_out = Re <p, ap> (FP64 sum)
 int schur_lo_v32(const qexstag_links_s *g, int prec, int par, float2 *ap, const float2 *p, float2 *t, double m2,
-                 double *dot_out) {
+                 double *dot_out, const Progress &progress) {
   const Geom &geo = g->l->g;
   DslashArgsLo A;
   A.g = geo;
@@ -743,12 +748,14 @@ int schur_lo_v32(const qexstag_links_s *g, int prec, int par, float2 *ap, const 
   A.out = t;
   A.ostride = geo.nh;
   A.b = 0.f;
+  A.progress = progress;
   auto sweeps = [&](auto nl) {
     constexpr int NL = decltype(nl)::value;
     if (prec == kF16)
       launch_lo<kF16, kF32, NL, 1, 0, 0, kF32>(A, 0);
     else
       launch_lo<kF32, kF32, NL, 1, 0, 0, kF32>(A, 0);
+    A.progress = Progress();
     A.po = par;
     A.xin = t;
     A.xs = p;
@@ -1067,7 +1074,6 @@ static int cg_mixed_t(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, d
                                                       red_partials(), red_tickets());
   note_launch();
   QS_LAUNCH_CHECK();
-  const int every = check_interval(nh);
   // Three kernels an iteration: the two half sweeps (the second leaves the
   // <p, Ap> and |Ap|^2 partials) and the fused update, which first tests the
   // previous update's |r|^2 (except right after the start or a reliable
@@ -1076,52 +1082,55 @@ static int cg_mixed_t(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, d
   int cur = 0;
   bool fresh = true;
   double *const R2[2] = {red_partials() + kMxR2, red_partials() + kMxR2b};
-  auto batch = [&]() -> int {
-    for (int i = 0; i < every; i++) {
-      int np = 0;
-      constexpr bool hs = PREC == kF16;  // <r, Ap> partials from half sweep 2
-      int rc2 = schur_lo(g, PREC, par, ap, P[cur], pt, m2, 4, st, nullptr, &np, hs ? rs : nullptr);
-      if (rc2) return rc2;
-      launch_pdl(mx_update_p_kernel<VP>, grid, kBlock, rs, xs, (const float2 *)ap, (const void *)P[cur],
-                 P[cur ^ 1], nh, st, (const double *)red_partials(), (const double *)(red_partials() + kMxApAp),
-                 np, (const double *)R2[cur], fresh ? 0 : grid, R2[cur ^ 1], cur,
-                 hs ? (const double *)(red_partials() + kMxRAp) : (const double *)nullptr);
-      note_launch();
-      cur ^= 1;
-      fresh = false;
-    }
-    QS_LAUNCH_CHECK();
-    return QEXSTAG_OK;
-  };
-  // The state is read one batch behind: the next batch is queued before the
-  // host waits for the snapshot.  When the snapshot shows the solve done or
-  // a reliable update due, that batch's kernels have returned at once
-  // (done / pending), and the update is queued after them.
-  StateSnapshot snap;
-  if ((rc = batch())) return rc;
+  Pace pace;
+  if ((rc = pace.start(ws, nh))) return rc;
+  Progress progress;
+  progress.word = pace.word;
+  progress.itn = &st->itn;
+  progress.stop = &st->done;
+  progress.pending = &st->pending;
+  progress.pin = &st->pin;
+  progress.epoch = &st->reliable;
   for (;;) {
-    if ((rc = snap.start(st, sizeof(MxState))) || (rc = batch()) || (rc = snap.wait(&hs, sizeof(MxState))))
+    unsigned long long seen;
+    if ((rc = pace.wait(&seen))) return rc;
+    if (pace.now(seen) && (seen & kPaceStop)) break;
+    if (pace.now(seen) && (seen & kPacePending)) {
+      // reliable update: fold the increment in, FP64 true residual; the
+      // direction corrected is the one the last update that ran read (the
+      // update that stopped wrote nothing, and the kernels queued after it
+      // return at once), and the iteration goes on from it
+      mx_flush_kernel<<<egrid, kBlock, 0, stream()>>>(x.p, xs, nh);
+      note_launch();
+      if ((rc = schur64(g, par, VecD{ax, nh}, cv(x), VecD{(double2 *)pt64, nh}, m2))) return rc;
+      cur = (seen & kPacePin) ? 1 : 0;
+      fresh = true;
+      mx_true_res_kernel<<<grid, kBlock, 0, stream()>>>(b.p, b.stride, ax, r, rs, nh, st, red_partials(),
+                                                        red_tickets());
+      mx_rp_kernel<VP><<<grid, kBlock, 0, stream()>>>(rs, P[cur], nh, st, red_partials(), red_tickets());
+      mx_p_reliable_kernel<VP><<<egrid, kBlock, 0, stream()>>>(rs, P[cur], nh, st);
+      mx_clear_pending_kernel<<<1, 1, 0, stream()>>>(st);
+      note_launch(4);
+      QS_LAUNCH_CHECK();
+      pace.next_epoch(seen);
+      continue;
+    }
+    int np = 0;
+    constexpr bool hs16 = PREC == kF16;  // <r, Ap> partials from half sweep 2
+    if ((rc = schur_lo(g, PREC, par, ap, P[cur], pt, m2, 4, st, nullptr, &np, hs16 ? rs : nullptr, progress)))
       return rc;
-    if (hs.done) break;
-    if (!hs.pending) continue;
-    // reliable update: fold the increment in, FP64 true residual; the
-    // direction corrected is the one the last update that ran read
-    // (P[hs.pin]: the update that stopped wrote nothing, and the kernels
-    // queued after it returned at once), and the iteration goes on from it
-    mx_flush_kernel<<<egrid, kBlock, 0, stream()>>>(x.p, xs, nh);
+    launch_pdl(mx_update_p_kernel<VP>, grid, kBlock, rs, xs, (const float2 *)ap, (const void *)P[cur], P[cur ^ 1], nh,
+               st, (const double *)red_partials(), (const double *)(red_partials() + kMxApAp), np,
+               (const double *)R2[cur], fresh ? 0 : grid, R2[cur ^ 1], cur,
+               hs16 ? (const double *)(red_partials() + kMxRAp) : (const double *)nullptr);
     note_launch();
-    if ((rc = schur64(g, par, VecD{ax, nh}, cv(x), VecD{(double2 *)pt64, nh}, m2))) return rc;
-    cur = hs.pin & 1;
-    fresh = true;
-    mx_true_res_kernel<<<grid, kBlock, 0, stream()>>>(b.p, b.stride, ax, r, rs, nh, st, red_partials(),
-                                                      red_tickets());
-    mx_rp_kernel<VP><<<grid, kBlock, 0, stream()>>>(rs, P[cur], nh, st, red_partials(), red_tickets());
-    mx_p_reliable_kernel<VP><<<egrid, kBlock, 0, stream()>>>(rs, P[cur], nh, st);
-    mx_clear_pending_kernel<<<1, 1, 0, stream()>>>(st);
-    note_launch(4);
     QS_LAUNCH_CHECK();
-    if ((rc = batch())) return rc;
+    cur ^= 1;
+    fresh = false;
+    pace.queued++;
   }
+  StateSnapshot snap;
+  if ((rc = snap.start(st, sizeof(MxState))) || (rc = snap.wait(&hs, sizeof(MxState)))) return rc;
   out->iterations = hs.itn;
   out->r2 = hs.b2 > 0 ? hs.r2 / hs.b2 : 0.0;
   out->nan = hs.nan;

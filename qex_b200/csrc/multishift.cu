@@ -132,6 +132,7 @@ struct MrhsArgs {
   CgmState *wst;
   double *partials;
   unsigned *ticket;
+  Progress progress;  // posted by this launch (the first half sweep)
 };
 
 // (re, im) += (ar, ai) (vr, vi) for both right-hand sides of a pair, nai = -ai
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A
   constexpr int kSets = 2 / G;
   __shared__ float4 part[kSets][4][G * NP][3][kMrhsSites];
   pdl_wait();
+  post_progress(A.progress);
   if (A.st->done) return;
   const Geom &g = A.g;
   const int nh = g.nh;
@@ -279,6 +281,7 @@ static void mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *
   A.ors = vs;
   A.b = 0.f;
   launch_pdl(dslash_mrhs_kernel<NL, 1, 0, 0, R12, NP, G>, grid, kBlock, A);
+  A.progress = Progress();
   A.po = par;
   A.xin = t;
   A.irs = vs;
@@ -303,7 +306,7 @@ static void mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, 
 
 // pair j of p at p + j*prs; of t and ap at j*3*nh
 static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p, size_t prs, float4 *t,
-                      float4 *ap, double m2, CgmState *st) {
+                      float4 *ap, double m2, CgmState *st, const Progress &progress) {
   const Geom &geo = g->l->g;
   MrhsArgs A;
   A.g = geo;
@@ -315,6 +318,7 @@ static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p
   A.wst = st;
   A.partials = red_partials();
   A.ticket = red_tickets();
+  A.progress = progress;
   const float b4 = (float)(4.0 * m2);
   if (g->nl == 8) {
     if (g->low.recon12)
@@ -602,9 +606,8 @@ static int read_cgm_head(const CgmState *d, CgmState *h) {
   return QEXSTAG_OK;
 }
 
-int check_interval(int nh);
 int schur_lo_v32(const qexstag_links_s *g, int prec, int par, float2 *ap, const float2 *p, float2 *t, double m2,
-                 double *dot_out);
+                 double *dot_out, const Progress &progress);
 int cg_mixed(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, double r2req, int maxits, int sloppy,
              double delta, CgOut *out, int *reliable);
 
@@ -650,29 +653,32 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
                           stream()));
   // grid rows share the GPU; kMaxRedBlocks slots per right-hand side
   const dim3 grid(std::min(grid_for(nh, kBlock, std::max(1, 8 / nvec)), kMaxRedBlocks), nvec);
-  const int every = check_interval(nh);
-  // one iteration's kernels after the operator's two half sweeps
+  Pace pace;
+  if ((rc = pace.start(ws, nh))) return rc;
+  Progress progress;
+  progress.word = pace.word;
+  progress.itn = &st->itn;
+  progress.stop = &st->done;
+  // an iteration: the operator's two half sweeps and the two updates
   auto solve = [&](auto v, auto schur) -> int {
     using VT = std::remove_pointer_t<decltype(v.r)>;
     cgm_init_kernel<VT><<<grid, kBlock, 0, stream()>>>(v, (const double2 *const *)pb, bstride, st, red_partials(),
                                                        red_tickets(), r2req);
     note_launch();
     QS_LAUNCH_CHECK();
-    int it = 0;
+    int rc2;
     for (;;) {
-      for (int i = 0; i < every; i++) {
-        int rc2 = schur(v);
-        if (rc2) return rc2;
-        it++;
-        launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, v, st, red_partials(), red_tickets());
-        launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, v, (const CgmState *)st, it);
-        note_launch(2);
-      }
+      unsigned long long seen;
+      if ((rc2 = pace.wait(&seen))) return rc2;
+      if (seen & kPaceStop) break;
+      if ((rc2 = schur(v))) return rc2;
+      pace.queued++;
+      launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, v, st, red_partials(), red_tickets());
+      launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, v, (const CgmState *)st, (int)pace.queued);
+      note_launch(2);
       QS_LAUNCH_CHECK();
-      int rc2 = read_cgm_head(st, &hs);
-      if (rc2) return rc2;
-      if (hs.done) break;
     }
+    if ((rc2 = read_cgm_head(st, &hs))) return rc2;
     constexpr int n = Lanes<VT>::n;
     const int egrid = grid_for(nh, kBlock, 8);
     for (int j = 0; j < nrhs; j++)
@@ -686,16 +692,16 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
   if (pairs) {
     CgmVecs<float4> v{(float4 *)pr, (float4 *)pap, (float4 *)pt, (float4 *)px, (float4 *)pp, nh, nshift, nvec};
     // p_0 of pair j lives at xs_off(j, 0)
-    rc = solve(v, [&](auto &w) { return schur_mrhs(g, par, nrhs, w.p, w.xs_off(1, 0), w.t, w.ap, m2, st); });
+    rc = solve(v, [&](auto &w) { return schur_mrhs(g, par, nrhs, w.p, w.xs_off(1, 0), w.t, w.ap, m2, st, progress); });
   } else if (fp32) {
     CgmVecs<float2> v{(float2 *)pr, (float2 *)pap, (float2 *)pt, (float2 *)px, (float2 *)pp, nh, nshift, 1};
-    rc = solve(v, [&](auto &w) { return schur_lo_v32(g, lprec, par, w.ap, w.p, w.t, m2, &st->pAp[0]); });
+    rc = solve(v, [&](auto &w) { return schur_lo_v32(g, lprec, par, w.ap, w.p, w.t, m2, &st->pAp[0], progress); });
   } else {
     if (nrhs != 1) return fail(QEXSTAG_ERR_ARG, "FP64 multi-shift takes one right-hand side");
     CgmVecs<double2> v{(double2 *)pr, (double2 *)pap, (double2 *)pt, (double2 *)px, (double2 *)pp, nh, nshift, 1};
     rc = solve(v, [&](auto &w) {
       return schur64(g, par, VecD{w.ap, nh}, CVecD{w.p, nh}, VecD{w.t, nh}, m2, kRedDot, nullptr, &st->done,
-                     &st->pAp[0]);
+                     &st->pAp[0], progress);
     });
   }
   if (rc) return rc;

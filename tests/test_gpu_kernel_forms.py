@@ -74,3 +74,23 @@ def test_shifted_systems_by_right_hand_sides(cuda, nrhs, naik):
             o.stagD2ee(ay, y, m * m + 0.25 * sg)
             assert np.linalg.norm((ay - b)[: V // 2]) <= 1.01e-10 * np.linalg.norm(b)
             assert not np.any(y[V // 2:])
+
+
+# a solve ends where it is told to, whatever was queued behind it: after 1, 2,
+# 7 (one more than are queued at a time) and 40 iterations
+@pytest.mark.parametrize("sloppy", [0, 1, 2])
+@pytest.mark.parametrize("maxits", [1, 2, 7, 40])
+def test_solve_stops_at_maxits(cuda, sloppy, maxits):
+    dims = (4, 6, 6, 10)
+    s = S.Staggered(S.Layout(dims), S.to_device_links(F.fat_naik_links(dims, 3)))
+    b = S.to_device_vector(F.even_source(dims, 4))
+    for _ in range(2):
+        sp = S.SolverParams(r2req=1e-24, maxits=maxits, sloppySolve=sloppy)
+        s.solveEE(cuda.zeros_like(b), b, 0.01, sp)
+        assert sp.iterations == maxits and sp.status == S.L.NOT_CONVERGED
+    sp = S.SolverParams(r2req=1e-20, sloppySolve=sloppy)
+    x = cuda.zeros_like(b)
+    s.solveEE(x, b, 0.3, sp)
+    assert sp.status == S.L.OK and sp.r2 <= 1e-20
+    s.solveEE(x, cuda.zeros_like(b), 0.3, sp)  # no source: no iterations
+    assert sp.iterations == 0 and not bool(x.any())
