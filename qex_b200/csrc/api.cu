@@ -24,6 +24,39 @@ int stagD_par(qexstag_links_s *g, int par, double2 *r, const double2 *x, double 
               double a);
 int rephase_links(qexstag_links_s *g, bool literal);
 
+void *ScratchPool::take(size_t bytes) {
+  std::lock_guard<std::mutex> lock(m_);
+  for (Buf &b : bufs_)
+    if (!b.used && b.bytes >= bytes) {
+      b.used = true;
+      return b.p;
+    }
+  // a free buffer that is too small makes way
+  for (size_t i = 0; i < bufs_.size(); i++)
+    if (!bufs_[i].used) {
+      cudaFree(bufs_[i].p);
+      bufs_.erase(bufs_.begin() + i);
+      break;
+    }
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  bufs_.push_back(Buf{p, bytes, true});
+  return p;
+}
+
+void ScratchPool::give(void *p) {
+  std::lock_guard<std::mutex> lock(m_);
+  for (Buf &b : bufs_)
+    if (b.p == p) b.used = false;
+}
+
+ScratchPool::~ScratchPool() {
+  for (Buf &b : bufs_) cudaFree(b.p);
+}
+
 int Workspace::get(int slot, size_t bytes, void **out) {
   auto it = bufs.find(slot);
   if (it != bufs.end() && it->second.first >= bytes) {

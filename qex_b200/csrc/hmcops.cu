@@ -11,8 +11,7 @@
 //    src/hmc/hmcAction.nim:248-255).
 // Fields are 4-direction link fields double2[4][9][V] (the library's link
 // layout).  The force gathers, per (site, direction), every plaquette and
-// 2x1 rectangle through the link as the product of its other links, with the
-// direction/parity-interleaved block order of the smearing sweeps.
+// 2x1 rectangle through the link, with the block order of the smearing sweeps.
 #include <algorithm>
 
 #include "smear.cuh"
@@ -133,7 +132,9 @@ __device__ __forceinline__ void tah(M3 &r, const M3 &m) {
   r.e[8].y -= t;
 }
 
-// F_mu(x) = projectTAH(U_mu(x) (cp sum P + cr sum R)), cp = plaq/3, cr = rect/3
+// F_mu(x) = projectTAH(U_mu(x) (cp sum P + cr sum R)), cp = plaq/3, cr = rect/3,
+// path by path: without rectangles (two products per path, nothing to share),
+// and where the scratch of the two-sweep form below cannot be had
 __global__ void __launch_bounds__(kSmBlock) gauge_force_kernel(Geom g, const double2 *__restrict__ u, double2 *f,
                                                                double cp, double cr) {
   SiteCtx c;
@@ -149,6 +150,293 @@ __global__ void __launch_bounds__(kSmBlock) gauge_force_kernel(Geom g, const dou
   m_nn(m, um, acc);
   tah(r, m);
   m_store(f + (size_t)mu * 9 * V, V, c.site, r);
+}
+
+// ---------------------------------------------------------------------------
+// The force in two sweeps.  With A_mu(x) the weighted sum of the open paths
+// beside U_mu(x), F_mu = projectTAH(U_mu A_mu^dag).  Every 2x1 rectangle is a
+// plaquette one of whose links is replaced by its own staple, so a first
+// sweep stores the two halves of every staple,
+//   Up_{mu,nu}(x) = U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
+//   Dn_{mu,nu}(x) = U_nu(x)^dag U_mu(x) U_nu(x+mu)      (a path beside U_mu(x+nu))
+// and the second adds, with W = U_mu(x+nu), V = U_nu(x+mu) above the link and
+// z = x-nu, W = U_mu(z), V = U_nu(z+mu) below it,
+//   U_nu(x) [cp W V^dag + cr Up_{mu,nu}(x+nu) V^dag + cr W Up_{nu,mu}(x+mu)^dag]
+//     + cr Dn_{nu,mu}(x-mu) W V^dag
+//   U_nu(z)^dag [cp W V + cr Dn_{mu,nu}(z-nu) V + cr W Up_{nu,mu}(z+mu)]
+//     + cr Dn_{nu,mu}(z-mu)^dag W V.
+// 42 3x3 products per link where following each path took 84.  The
+// sweeps go through the lattice in slabs of time slices, with two slices
+// below and one above of their own, so that the 24 fields of 144 B per site
+// take at most kGaugeScratch (any lattice up to 32^4 is one slab).
+//
+// Bound by what L2 delivers (36 matrices a link) and FP64 issue.  24^4: 255 us
+// for the halves and 651 us for the force (255 registers and 8 warps an SM; 758
+// us at 168 registers, which spill), against 1670 us path by path.
+// ---------------------------------------------------------------------------
+
+struct GaugeArgs {
+  Geom g;
+  const double2 *u;
+  double2 *f;
+  double2 *up, *dn;  // [4][3][9][2 nk]: parity blocks of the slab's nk half sites
+  int k0, nk;        // the slab: half sites k0 .. k0 + nk - 1, periodic
+  int o0, on;        // the half sites whose force this launch forms
+  double cp, cr;
+};
+
+// Block b works on direction b % 4 and both parities of 64 half sites
+// (start .. start + n - 1, periodic) of the list.
+__device__ __forceinline__ bool site_of_slab(const Geom &g, SiteCtx &c, int start, int n) {
+  const int b = blockIdx.x, w = threadIdx.x >> 5;
+  c.mu = b & 3;
+  c.par = w & 1;
+  const int i = (b >> 2) * (kSmBlock / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  if (i >= n) return false;
+  int k = start + i;
+  if (k >= g.nh) k -= g.nh;
+  c.site = c.par * g.nh + k;
+  site_coords(g, c.par, k, c.x, c.lex);
+  return true;
+}
+inline int slab_grid(int n) { return 4 * ((n + kSmBlock / 2 - 1) / (kSmBlock / 2)); }
+
+// place of a site in the slab's fields
+__device__ __forceinline__ int in_slab(const GaugeArgs &A, int site) {
+  const int par = site >= A.g.nh ? 1 : 0;
+  int d = site - par * A.g.nh - A.k0;
+  if (d < 0) d += A.g.nh;
+  return par * A.nk + d;
+}
+
+__device__ __forceinline__ void ld_row(double2 r[3], const double2 *__restrict__ F, size_t V, int s, int i) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) r[k] = __ldg(F + (size_t)(3 * i + k) * V + s);
+}
+__device__ __forceinline__ void ld_col(double2 r[3], const double2 *__restrict__ F, size_t V, int s, int k) {
+#pragma unroll
+  for (int i = 0; i < 3; i++) r[i] = __ldg(F + (size_t)(3 * i + k) * V + s);
+}
+// out_j += (row r) m or (row r) m^dag
+__device__ __forceinline__ void row_nn(double2 *out, const double2 r[3], const M3 &m) {
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) out[j] = cmadd(out[j], r[k], m.e[3 * k + j]);
+}
+__device__ __forceinline__ void row_nd(double2 *out, const double2 r[3], const M3 &m) {
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) out[j] = cjmadd(out[j], m.e[3 * j + k], r[k]);
+}
+__device__ __forceinline__ void scale3(double2 r[3], double a) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    r[k].x *= a;
+    r[k].y *= a;
+  }
+}
+// acc += (column c of a matrix) (row r), or with conj(c)
+__device__ __forceinline__ void outer_nn(M3 &acc, const double2 c[3], const double2 *r) {
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) acc.e[3 * i + j] = cmadd(acc.e[3 * i + j], c[i], r[j]);
+}
+__device__ __forceinline__ void outer_dn(M3 &acc, const double2 c[3], const double2 *r) {
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) acc.e[3 * i + j] = cjmadd(acc.e[3 * i + j], c[i], r[j]);
+}
+
+__global__ void __launch_bounds__(kSmBlock, 3) gauge_halves_kernel(const GaugeArgs A) {
+  SiteCtx c;
+  const Geom &g = A.g;
+  if (!site_of_slab(g, c, A.k0, A.nk)) return;
+  const int mu = c.mu;
+  const size_t V = (size_t)g.V, N = (size_t)2 * A.nk;
+  const int here = in_slab(A, c.site);
+  const double2 *Um = A.u + (size_t)mu * 9 * V;
+  const int s_pm = disp1(g, c.x, c.lex, c.par, mu, 1);
+#pragma unroll 1
+  for (int j = 0; j < 3; j++) {
+    const int nu = other_dir(mu, j);
+    const double2 *Un = A.u + (size_t)nu * 9 * V;
+    const int s_pn = disp1(g, c.x, c.lex, c.par, nu, 1);
+    double2 *up = A.up + (size_t)(mu * 3 + j) * 9 * N + here, *dn = A.dn + (size_t)(mu * 3 + j) * 9 * N + here;
+    M3 v, t;
+    m_load(v, Un, V, s_pm);
+    m_zero(t);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      double2 r[3];
+      ld_row(r, Um, V, s_pn, i);
+      row_nd(t.e + 3 * i, r, v);  // U_mu(x+nu) V^dag
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      double2 r[3], o[3] = {};
+      ld_row(r, Un, V, c.site, i);
+      row_nn(o, r, t);
+#pragma unroll
+      for (int k = 0; k < 3; k++) up[(size_t)(3 * i + k) * N] = o[k];
+    }
+    m_zero(t);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      double2 r[3];
+      ld_row(r, Um, V, c.site, i);
+      row_nn(t.e + 3 * i, r, v);  // U_mu(x) V
+    }
+    m_zero(v);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      double2 r[3];
+      ld_row(r, Un, V, c.site, k);
+      outer_dn(v, r, t.e + 3 * k);
+    }
+#pragma unroll
+    for (int e = 0; e < 9; e++) dn[(size_t)e * N] = v.e[e];
+  }
+}
+
+__global__ void __launch_bounds__(kSmBlock, 2) gauge_rect_force_kernel(const GaugeArgs A) {
+  SiteCtx c;
+  const Geom &g = A.g;
+  if (!site_of_slab(g, c, A.o0, A.on)) return;
+  const int mu = c.mu;
+  const size_t V = (size_t)g.V, N = (size_t)2 * A.nk;
+  const double2 *Um = A.u + (size_t)mu * 9 * V;
+  const double cp = A.cp, cr = A.cr;
+  M3 acc;
+  m_zero(acc);
+  const int s_pm = disp1(g, c.x, c.lex, c.par, mu, 1);
+  const int l_pm = in_slab(A, s_pm), l_mm = in_slab(A, disp1(g, c.x, c.lex, c.par, mu, -1));
+#pragma unroll 1
+  for (int j = 0; j < 3; j++) {
+    const int nu = other_dir(mu, j);
+    const double2 *Un = A.u + (size_t)nu * 9 * V;
+    const double2 *up_mn = A.up + (size_t)(mu * 3 + j) * 9 * N, *dn_mn = A.dn + (size_t)(mu * 3 + j) * 9 * N;
+    const int jm = nu * 3 + other_index(nu, mu);
+    const double2 *up_nm = A.up + (size_t)jm * 9 * N, *dn_nm = A.dn + (size_t)jm * 9 * N;
+    M3 v, P, K;
+    // above the link
+    {
+      const int s_pn = disp1(g, c.x, c.lex, c.par, nu, 1);
+      const int l_pn = in_slab(A, s_pn);
+      m_load(v, Un, V, s_pm);
+      m_zero(P);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double2 r[3];
+        ld_row(r, Um, V, s_pn, i);
+        row_nd(P.e + 3 * i, r, v);
+#pragma unroll
+        for (int k = 0; k < 3; k++) K.e[3 * i + k] = make_double2(cp * P.e[3 * i + k].x, cp * P.e[3 * i + k].y);
+        ld_row(r, up_mn, N, l_pn, i);
+        scale3(r, cr);
+        row_nd(K.e + 3 * i, r, v);
+      }
+      m_load(v, up_nm, N, l_pm);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double2 r[3];
+        ld_row(r, Um, V, s_pn, i);
+        scale3(r, cr);
+        row_nd(K.e + 3 * i, r, v);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        double2 r[3];
+        ld_col(r, Un, V, c.site, k);
+        outer_nn(acc, r, K.e + 3 * k);
+        ld_col(r, dn_nm, N, l_mm, k);
+        scale3(r, cr);
+        outer_nn(acc, r, P.e + 3 * k);
+      }
+    }
+    // below it
+    {
+      const int z = disp1(g, c.x, c.lex, c.par, nu, -1), zpm = disp2(g, c.x, c.lex, c.par, nu, -1, mu, 1);
+      const int l_2 = in_slab(A, disp1(g, c.x, c.lex, c.par, nu, -2));
+      const int l_zpm = in_slab(A, zpm), l_zmm = in_slab(A, disp2(g, c.x, c.lex, c.par, nu, -1, mu, -1));
+      m_load(v, Un, V, zpm);
+      m_zero(P);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double2 r[3];
+        ld_row(r, Um, V, z, i);
+        row_nn(P.e + 3 * i, r, v);
+#pragma unroll
+        for (int k = 0; k < 3; k++) K.e[3 * i + k] = make_double2(cp * P.e[3 * i + k].x, cp * P.e[3 * i + k].y);
+        ld_row(r, dn_mn, N, l_2, i);
+        scale3(r, cr);
+        row_nn(K.e + 3 * i, r, v);
+      }
+      m_load(v, up_nm, N, l_zpm);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double2 r[3];
+        ld_row(r, Um, V, z, i);
+        scale3(r, cr);
+        row_nn(K.e + 3 * i, r, v);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        double2 r[3];
+        ld_row(r, Un, V, z, k);
+        outer_dn(acc, r, K.e + 3 * k);
+        ld_row(r, dn_nm, N, l_zmm, k);
+        scale3(r, cr);
+        outer_dn(acc, r, P.e + 3 * k);
+      }
+    }
+  }
+  M3 um, m;
+  m_load(um, Um, V, c.site);
+  m_nd(m, um, acc);
+  tah(um, m);
+  m_store(A.f + (size_t)mu * 9 * V, V, c.site, um);
+}
+
+constexpr size_t kGaugeScratch = (size_t)4 << 30;
+
+// the plaquette and rectangle force through the slabs; QEXSTAG_ERR_ALLOC (with
+// nothing launched) where their scratch cannot be had
+static int rect_force_dev(qexstag_layout_s *l, const double2 *u, double2 *f, double cp, double cr) {
+  const Geom &g = l->g;
+  const int T = g.L[3], sh = g.nh / T;  // half sites of a time slice
+  const size_t slice = (size_t)24 * 9 * sizeof(double2) * 2 * sh;
+  int n = T;  // slices of force per slab
+  if (slice * T > kGaugeScratch) n = std::max(1, std::min(T, (int)(kGaugeScratch / slice) - 3));
+  const int held = std::min(T, n + 3);  // slices of scratch
+  if (n == 1 && held == 4 && T > 4 && slice * held > kGaugeScratch) return QEXSTAG_ERR_ALLOC;
+  void *p = l->scratch.take(slice * held);
+  if (!p) return QEXSTAG_ERR_ALLOC;
+  GaugeArgs A;
+  A.g = g;
+  A.u = u;
+  A.f = f;
+  A.nk = held * sh;
+  A.up = (double2 *)p;
+  A.dn = A.up + (size_t)12 * 9 * 2 * A.nk;
+  A.cp = cp;
+  A.cr = cr;
+  for (int t = 0; t < T; t += n) {
+    const int here = std::min(n, T - t);
+    A.k0 = held == T ? 0 : ((t - 2 + T) % T) * sh;
+    A.o0 = t * sh;
+    A.on = here * sh;
+    gauge_halves_kernel<<<slab_grid(A.nk), kSmBlock, 0, stream()>>>(A);
+    gauge_rect_force_kernel<<<slab_grid(A.on), kSmBlock, 0, stream()>>>(A);
+    note_launch(2);
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream());
+  l->scratch.give(p);
+  return e == cudaSuccess ? QEXSTAG_OK : cuda_fail(e, "gauge_force");
 }
 
 // sum_{x, mu>nu} Re Tr P and sum_{x, mu!=nu} Re Tr R (long side mu), each
@@ -445,9 +733,14 @@ int qexstag_gauge_force(qexstag_layout *l, const qexstag_gauge_coefs *c, const d
   const Geom &g = l->g;
   Field4 U, Fo;
   if ((rc = field_in(g, u, mem, true, U)) || (rc = field_in(g, f, mem, false, Fo))) return rc;
-  gauge_force_kernel<<<sweep_grid(g), kSmBlock, 0, stream()>>>(g, U.dev, Fo.dev, c->plaq / 3.0, c->rect / 3.0);
-  note_launch();
-  QS_LAUNCH_CHECK();
+  rc = c->rect != 0.0 ? rect_force_dev(l, U.dev, Fo.dev, c->plaq / 3.0, c->rect / 3.0) : QEXSTAG_ERR_ALLOC;
+  if (rc == QEXSTAG_ERR_ALLOC) {
+    gauge_force_kernel<<<sweep_grid(g), kSmBlock, 0, stream()>>>(g, U.dev, Fo.dev, c->plaq / 3.0, c->rect / 3.0);
+    note_launch();
+    QS_LAUNCH_CHECK();
+  } else if (rc) {
+    return rc;
+  }
   if ((rc = field_out(Fo))) return rc;
   QS_CUDA(cudaStreamSynchronize(stream()));
   return QEXSTAG_OK;

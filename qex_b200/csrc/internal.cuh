@@ -9,7 +9,9 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/qexstag.h"
 
@@ -335,8 +337,31 @@ inline int grid_for(long n, int block = kBlock, int per_sm = 8) {
 
 }  // namespace qs
 
+namespace qs {
+// Device buffers kept with a layout between calls.  A call holds one for its
+// duration (every entry point that takes one waits for its kernels before it
+// returns), so threads that call with one layout at the same time, on
+// whatever streams, get one each; all are freed with the layout.
+class ScratchPool {
+ public:
+  void *take(size_t bytes);  // null when it cannot be had
+  void give(void *p);
+  ~ScratchPool();
+
+ private:
+  struct Buf {
+    void *p;
+    size_t bytes;
+    bool used;
+  };
+  std::mutex m_;
+  std::vector<Buf> bufs_;
+};
+}  // namespace qs
+
 // handles
 struct qexstag_layout_s {
   qs::Geom g;
   int device;
+  qs::ScratchPool scratch;
 };

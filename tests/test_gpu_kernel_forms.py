@@ -6,6 +6,7 @@ import pytest
 
 from oracle import oracle as O
 from qex_b200 import fields as F
+from qex_b200 import md as MD
 from qex_b200 import smear as SM
 from qex_b200 import stag as S
 
@@ -94,3 +95,36 @@ def test_solve_stops_at_maxits(cuda, sloppy, maxits):
     assert sp.status == S.L.OK and sp.r2 <= 1e-20
     s.solveEE(x, cuda.zeros_like(b), 0.3, sp)  # no source: no iterations
     assert sp.iterations == 0 and not bool(x.any())
+
+
+# the force with rectangles in two sweeps: 720 half sites are 11 1/4 blocks
+def test_rectangle_force_remainders(cuda):
+    dims = (4, 6, 6, 10)
+    lay, u = S.Layout(dims), F.gauge_warm(dims, 0.5, 6)
+    ud = S.to_device_links(u)
+    f = cuda.empty_like(ud)
+    act = MD.GaugeAction(lay, 5.6, -1.0 / 12.0)
+    act.force(ud, f)
+    assert rel(S.to_host_links(f), O.gauge_force(dims, u, act.c.plaq, act.c.rect)) < 1e-12
+
+
+# and through more than one slab of time slices: 48 slices of 32^3 take two,
+# the first of them with its lower neighbours beyond the periodic boundary.
+# The links repeat after 24 slices, which are one slab by themselves, so the
+# force must repeat too, bit for bit.
+def test_rectangle_force_slabs(cuda):
+    torch = cuda
+    half, full = (32, 32, 32, 24), (32, 32, 32, 48)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    u = torch.view_as_complex(torch.randn((4, 3, 3, F.volume(half), 2), dtype=torch.float64, device="cuda",
+                                          generator=gen))
+    x = F.coords(full)
+    x[:, 3] %= 24
+    place = torch.from_numpy(F.index_of(half, x)).to("cuda")
+    one, two = MD.GaugeAction(S.Layout(half), 5.6, -0.331), MD.GaugeAction(S.Layout(full), 5.6, -0.331)
+    f1 = torch.empty_like(u)
+    one.force(u, f1)
+    u2 = u.index_select(3, place)
+    f2 = torch.empty_like(u2)
+    two.force(u2, f2)
+    assert torch.equal(f2, f1.index_select(3, place))
