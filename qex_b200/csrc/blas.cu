@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 template <int K>
-static int reduce(CVecD x, CVecD y, int n, double *host) {
-  double *res = red_results();
+static int reduce(CVecD x, CVecD y, int n, double *host, double *dev = nullptr) {
+  double *res = dev ? dev : red_results();
   int grid = grid_for(n, kBlock, 4);
   reduce_kernel<K><<<grid, kBlock, 0, stream()>>>(x.p, x.stride, y.p, y.stride, n, red_partials(),
                                                  red_tickets(), res);
@@ -142,6 +142,7 @@ static int reduce(CVecD x, CVecD y, int n, double *host) {
 }
 
 int vnorm2(CVecD x, int n, double *host) { return reduce<kNorm2>(x, kNone, n, host); }
+int vnorm2_dev(CVecD x, int n, double *dev) { return reduce<kNorm2>(x, kNone, n, nullptr, dev); }
 int vredot(CVecD x, CVecD y, int n, double *host) { return reduce<kRedot>(x, y, n, host); }
 int vdiffnorm2(CVecD a, CVecD b, int n, double *host) { return reduce<kDiffNorm2>(a, b, n, host); }
 

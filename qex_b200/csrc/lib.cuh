@@ -124,6 +124,7 @@ int vaxpby(VecD y, double a, CVecD x, double b, int n);  // y = a x + b y
 int vsub(VecD y, CVecD a, CVecD b, int n);           // y = a - b
 // reductions to a device double (result) and, when host != nullptr, to host
 int vnorm2(CVecD x, int n, double *host);
+int vnorm2_dev(CVecD x, int n, double *dev);  // to a device double of the caller's, no wait
 int vredot(CVecD x, CVecD y, int n, double *host);
 // |a - b|^2 (no write)
 int vdiffnorm2(CVecD a, CVecD b, int n, double *host);

@@ -128,3 +128,23 @@ def test_rectangle_force_slabs(cuda):
     f2 = torch.empty_like(u2)
     two.force(u2, f2)
     assert torch.equal(f2, f1.index_select(3, place))
+
+
+# batches: one problem, an odd set count (720 even sites are 22 1/2 sets of 32),
+# and 70 problems (more than the norms read back at a time)
+@pytest.mark.parametrize("shapes", [[(4, 4, 4, 4)], [(4, 6, 6, 10), (4, 4, 4, 4), (6, 4, 4, 6)], [(4, 4, 4, 4)] * 70])
+def test_batch_partitions(cuda, shapes):
+    ops, bs, ms, gs = [], [], [], []
+    for j, dims in enumerate(shapes):
+        gs.append(F.naive_links(dims, 0.3, 3 + j % 5))
+        ops.append(S.Staggered(S.Layout(dims), S.to_device_links(gs[-1])))
+        bs.append(F.even_source(dims, 40 + j))
+        ms.append(0.1 + 0.02 * (j % 7))
+    xs = [S.to_device_vector(np.zeros_like(b)) for b in bs]
+    out = S.solve_batched(ops, xs, [S.to_device_vector(b) for b in bs], ms, S.SolverParams(r2req=1e-20))
+    assert (out["r2"] <= 1e-20).all()
+    for dims, g, m, b, x in zip(shapes, gs, ms, bs, xs):
+        o = O.Oracle(dims, g)
+        x, ax = S.to_host_vector(x), o.vec()
+        o.stagD2ee(ax, x, m * m)
+        assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
