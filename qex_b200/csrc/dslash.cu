@@ -45,7 +45,47 @@ struct DslashArgs64 {
   int k0, n1, k2, nsites;
   int rowlen, pitch;
   Progress progress;  // posted by this launch (a solve's first half sweep)
+  CgFused cg;         // fused CG (CG > 0)
 };
+
+// Start of a fused CG iteration, in every block: the sum of the previous
+// iteration's |r|^2, QEX's loop test (cg.nim:174) and beta.  All blocks add
+// the same partials in the same order; block 0 records.  What other blocks
+// read is not written here: rz alternates between two fields, and a block
+// that finds done already set leaves as it would have by its own test.
+__device__ __forceinline__ bool cg_begin(const CgFused &F, double *beta) {
+  __shared__ double sh[32], sh_beta;
+  __shared__ int sh_go;
+  CgState *st = F.st;
+  const int par = F.it & 1;
+  if (__syncthreads_or(st->done)) return false;  // one answer for the block: block 0 of this launch may be setting it
+  double v[1] = {0.0};
+  if (F.it > 0) {
+    for (int i = threadIdx.x; i < F.nr2; i += blockDim.x) v[0] += __ldcg(F.r2part + i);
+    block_sum<1>(v, sh);
+  }
+  if (threadIdx.x == 0) {
+    const double r2 = F.it > 0 ? v[0] : st->b2;
+    const bool bad = isnan(r2);
+    const bool go = F.it == 0 || (!bad && F.it < st->maxits && r2 > st->r2stop);
+    sh_go = go;
+    sh_beta = F.it > 0 ? r2 / st->rzs[par] : 0.0;
+    if (blockIdx.x == 0) {
+      st->r2 = r2;
+      st->itn = F.it;
+      if (go) {
+        st->beta = sh_beta;
+        st->rzs[par ^ 1] = r2;
+      } else {
+        st->nan = bad;
+        st->done = 1;
+      }
+    }
+  }
+  __syncthreads();
+  *beta = sh_beta;
+  return sh_go;
+}
 
 // j-th output site of the launch, as an index of the parity block
 __device__ __forceinline__ int out_site(const DslashArgs64 &A, int j) {
@@ -178,13 +218,25 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
 constexpr int kSplitSites = 32;
 constexpr int kSplitWarps = kBlock / 32;
 
-template <int NL, int HOP, int INIT, int RED>
+// CG > 0: the sweeps of a fused CG iteration.  CG = 1, the first, forms its
+// input r + beta p at the neighbours; CG = 2, the second, forms p at its own
+// sites and leaves each block's part of <p, Ap>.
+template <int NL, int HOP, int INIT, int RED, int CG = 0>
 __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs64 A) {
   constexpr int kTerms = 2 * NL, kPer = kTerms / kSplitWarps;
   __shared__ double2 term[kTerms][3][kSplitSites];
   pdl_wait();
-  post_progress(A.progress);
-  if (A.done != nullptr && *A.done) return;
+  double beta = 0.0;
+  if (CG == 1) {
+    if (!cg_begin(A.cg, &beta)) return;
+  } else if (CG == 2) {
+    post_progress(A.progress);
+    if (A.cg.st->done) return;
+    beta = A.cg.st->beta;
+  } else {
+    post_progress(A.progress);
+    if (A.done != nullptr && *A.done) return;
+  }
   const Geom &g = A.g;
   const int nh = g.nh;
   const size_t V = (size_t)g.V;
@@ -192,6 +244,17 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
   const size_t out_base = (size_t)A.po * nh;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double dot = 0.0;
+  auto gather = [&](int n, double2 v[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + n);
+    if (CG == 1 && A.cg.it > 0) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double2 pv = ldg(A.cg.p + (size_t)c * nh + n);
+        v[c] = make_double2(fma(beta, pv.x, v[c].x), fma(beta, pv.y, v[c].y));
+      }
+    }
+  };
   for (int j0 = blockIdx.x * kSplitSites; j0 < A.nsites; j0 += gridDim.x * kSplitSites) {
     const bool on = j0 + lane < A.nsites;
     const int k = out_site(A, on ? j0 + lane : j0);
@@ -207,8 +270,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
         const int jf = (lex + lex_step(g, x, mu, len)) >> 1;
 #pragma unroll
         for (int e = 0; e < 9; e++) m[e] = ldlink(ul + (size_t)e * V + out_base + k);
-#pragma unroll
-        for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + jf);
+        gather(jf, v);
 #pragma unroll
         for (int i = 0; i < 3; i++) {
           t[i] = make_double2(0.0, 0.0);
@@ -219,8 +281,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
         const int jb = (lex + lex_step(g, x, mu, -len)) >> 1;
 #pragma unroll
         for (int e = 0; e < 9; e++) m[e] = ldlink(ul + (size_t)e * V + in_base + jb);
-#pragma unroll
-        for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + jb);
+        gather(jb, v);
 #pragma unroll
         for (int i = 0; i < 3; i++) {
           t[i] = make_double2(0.0, 0.0);
@@ -237,6 +298,14 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
       double2 acc = make_double2(0.0, 0.0), xsv = acc;
       if (INIT > 0) {
         xsv = __ldcg(A.xs + (size_t)c * A.sstride + k);
+        if (CG == 2) {  // xs is r
+          double2 *p = A.cg.p + (size_t)c * nh + k;
+          if (A.cg.it > 0) {
+            const double2 pv = __ldcg(p);
+            xsv = make_double2(fma(beta, pv.x, xsv.x), fma(beta, pv.y, xsv.y));
+          }
+          *p = xsv;
+        }
         acc = make_double2(A.b * xsv.x, A.b * xsv.y);
       }
       if (INIT == 2) {
@@ -257,14 +326,21 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
       }
       const double2 o = make_double2(A.c * acc.x, A.c * acc.y);
       A.out[(size_t)c * A.ostride + k] = o;
-      if (RED != kRedNone) {
+      if (RED != kRedNone || CG == 2) {
         dot = fma(xsv.x, o.x, dot);
         dot = fma(xsv.y, o.y, dot);
       }
     }
     __syncthreads();
   }
-  if (RED != kRedNone) reduce_pap<RED>(A, dot);
+  if (CG == 2) {
+    __shared__ double sh[32];
+    double v[1] = {dot};
+    block_sum<1>(v, sh);
+    if (threadIdx.x == 0) A.cg.pap[blockIdx.x] = v[0];
+  } else if (RED != kRedNone) {
+    reduce_pap<RED>(A, dot);
+  }
 }
 
 // Sites per launch up to which a half sweep spreads each site over a block's
@@ -404,6 +480,46 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
   const int init = xs.p ? 1 : 0;
   const int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, kRedNone) : dispatch64<4>(A, hop, init, kRedNone);
   if (rc) return rc;
+  QS_LAUNCH_CHECK();
+  return QEXSTAG_OK;
+}
+
+bool cg_fused_fits(const qexstag_links_s *gl) {
+  return gl->l->g.nh <= (gl->nl == 8 ? kSplitMax<8> : kSplitMax<4>);
+}
+
+// the two half sweeps of a fused CG iteration; *npap: the <p, Ap> partials
+int schur64_fused(const qexstag_links_s *gl, int par, const CgFused &F, double m2, const Progress &progress, int *npap) {
+  const Geom &g = gl->l->g;
+  DslashArgs64 A = {};
+  A.g = g;
+  A.u = gl->u64;
+  A.n1 = A.nsites = g.nh;
+  A.cg = F;
+  A.c = 1.0;
+  const int grid = std::min((g.nh + kSplitSites - 1) / kSplitSites, num_sms() * 3);
+  A.po = 1 - par;
+  A.xin = F.r;
+  A.istride = g.nh;
+  A.out = F.t;
+  A.ostride = g.nh;
+  if (gl->nl == 8)
+    launch_pdl(dslash64_split_kernel<8, 1, 0, kRedNone, 1>, grid, kBlock, A);
+  else
+    launch_pdl(dslash64_split_kernel<4, 1, 0, kRedNone, 1>, grid, kBlock, A);
+  A.po = par;
+  A.xin = F.t;
+  A.xs = F.r;
+  A.sstride = g.nh;
+  A.out = F.ap;
+  A.b = 4.0 * m2;
+  A.progress = progress;  // its work covers the report's wait, the other kernels' is shorter
+  if (gl->nl == 8)
+    launch_pdl(dslash64_split_kernel<8, -1, 1, kRedNone, 2>, grid, kBlock, A);
+  else
+    launch_pdl(dslash64_split_kernel<4, -1, 1, kRedNone, 2>, grid, kBlock, A);
+  note_launch(2);
+  *npap = grid;
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
 }

@@ -250,6 +250,7 @@ struct CgState {
   int nan;
   int reliable;   // mixed: number of reliable updates done
   int pad[3];
+  double rzs[2];  // fused CG: rz of the iteration, alternating (CgFused)
 };
 
 // A running solve's report to the host, one 64-bit word in pinned memory:

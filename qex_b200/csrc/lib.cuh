@@ -102,6 +102,21 @@ int cg_mixed_domain(const MxDomain &D, double m2, const double2 *b, double2 *x, 
 // stagDN (mrhs.cu): r[i] (parity po) = m x[i] + (2D) x[i], i < n
 int dslashN64(const qexstag_links_s *gl, int po, int n, double2 *const *r, int rstride, const double2 *const *x,
               int xstride, double m);
+// One iteration's operator of the fused CG (cg64 on lattices whose half sweeps
+// spread a site over warps): the two half sweeps form p = r + beta p
+// themselves, and the sums of one kernel are finished by the blocks of the
+// next.  it counts iterations from 0.
+struct CgFused {
+  const double2 *r;  // [3][nh]
+  double2 *p, *ap, *t;
+  CgState *st;
+  const double *r2part;  // |r|^2 partials of the previous iteration, nr2 of them
+  int nr2;
+  double *pap;  // <p, Ap> partials of this one
+  int it;
+};
+bool cg_fused_fits(const qexstag_links_s *gl);
+int schur64_fused(const qexstag_links_s *gl, int par, const CgFused &F, double m2, const Progress &progress, int *npap);
 // Schur operator on parity par: r = 4 m2 x - (2D)_{par,q} (2D)_{q,par} x,
 // with t (q block) the temporary; red kRedCgPAp/kRedDot accumulate Re<x, r>.
 int schur64(const qexstag_links_s *g, int par, VecD r, CVecD x, VecD t, double m2,
