@@ -20,6 +20,7 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
 int solve_multishift(qexstag_links_s *g, int nmass, double2 *const *xs, const double2 *b,
                      const double *ms, const qexstag_solver_params *p, qexstag_solver_stats *st);
 int apply_D(qexstag_links_s *g, double2 *r, const double2 *x, double m, double sc);
+int stagD_all(qexstag_links_s *g, double2 *r, const double2 *x, double m, double sc, double a);
 int stagD_par(qexstag_links_s *g, int par, double2 *r, const double2 *x, double m, double sc,
               double a);
 int rephase_links(qexstag_links_s *g, bool literal);
@@ -618,8 +619,7 @@ static int stagD_api(qexstag_links *g, int subset, double *r, const double *x, d
     if ((rc = stage_in(g, kSlotOut0, r, mem, &dr_in))) return rc;
   }
   if (subset == 2) {
-    if ((rc = stagD_par(g, 0, dr, dx, m, sc, a))) return rc;
-    if ((rc = stagD_par(g, 1, dr, dx, m, sc, a))) return rc;
+    if ((rc = stagD_all(g, dr, dx, m, sc, a))) return rc;
   } else {
     if ((rc = stagD_par(g, subset, dr, dx, m, sc, a))) return rc;
   }

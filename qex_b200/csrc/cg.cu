@@ -363,10 +363,20 @@ int stagD_par(qexstag_links_s *g, int par, double2 *r, const double2 *x, double 
                   block((const double2 *)r, geo, par), aa, bb, h, +1, init);
 }
 
+// stagD on all sites
+int stagD_all(qexstag_links_s *g, double2 *r, const double2 *x, double m, double sc, double a) {
+  if (r == x) {  // in place: one parity after the other
+    int rc = stagD_par(g, 0, r, x, m, sc, a);
+    return rc ? rc : stagD_par(g, 1, r, x, m, sc, a);
+  }
+  const double h = 0.5 * sc;
+  const double aa = a / h, bb = m / h;
+  const int init = (aa == 0.0 && bb == 0.0) ? 0 : (aa == 0.0 ? 1 : 2);
+  return dslash64_both(g, r, x, r, aa, bb, h, init);
+}
+
 int apply_D(qexstag_links_s *g, double2 *r, const double2 *x, double m, double sc) {
-  int rc = stagD_par(g, 0, r, x, m, sc, 0.0);
-  if (rc) return rc;
-  return stagD_par(g, 1, r, x, m, sc, 0.0);
+  return stagD_all(g, r, x, m, sc, 0.0);
 }
 
 static int solve_xx_internal(qexstag_links_s *g, int par, double2 *y, const double2 *b, double m,

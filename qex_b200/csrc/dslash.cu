@@ -44,6 +44,9 @@ struct DslashArgs64 {
   // instead nsites / rowlen runs of rowlen sites, pitch apart, from k0
   int k0, n1, k2, nsites;
   int rowlen, pitch;
+  // both parities in one launch, even blocks on even sites: po is unused and
+  // the fields' pointers are those of the whole lattice
+  int both;
   Progress progress;  // posted by this launch (a solve's first half sweep)
   CgFused cg;         // fused CG (CG > 0)
 };
@@ -121,13 +124,17 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
   const Geom &g = A.g;
   const int nh = g.nh;
   const size_t V = (size_t)g.V;
-  const size_t in_base = (size_t)(1 - A.po) * nh;
-  const size_t out_base = (size_t)A.po * nh;
+  const int po = A.both ? (int)(blockIdx.x & 1) : A.po;
+  const int block = A.both ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> A.both;
+  const size_t in_base = (size_t)(1 - po) * nh;
+  const size_t out_base = (size_t)po * nh;
+  const size_t in_off = A.both ? in_base : 0, out_off = A.both ? out_base : 0;
+  const double2 *__restrict__ xin = A.xin + in_off;
   double dot = 0.0;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < A.nsites; j += gridDim.x * blockDim.x) {
+  for (int j = block * blockDim.x + threadIdx.x; j < A.nsites; j += blocks * blockDim.x) {
     const int k = out_site(A, j);
     int x[4], lex;
-    site_coords(g, A.po, k, x, lex);
+    site_coords(g, po, k, x, lex);
     double2 acc[3];
     double2 xsv[3];
     if (INIT == 0) {
@@ -136,13 +143,13 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
     } else {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        xsv[c] = __ldcg(A.xs + (size_t)c * A.sstride + k);
+        xsv[c] = __ldcg(A.xs + (size_t)c * A.sstride + out_off + k);
         acc[c] = make_double2(A.b * xsv[c].x, A.b * xsv[c].y);
       }
       if (INIT == 2) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          double2 rv = __ldcg(A.rin + (size_t)c * A.rstride + k);
+          double2 rv = __ldcg(A.rin + (size_t)c * A.rstride + out_off + k);
           acc[c].x = fma(A.a, rv.x, acc[c].x);
           acc[c].y = fma(A.a, rv.y, acc[c].y);
         }
@@ -156,11 +163,11 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
       const double2 *ul = A.u + (size_t)l * 9 * V;
       double2 v[3], w[3], uf[9], ub[9];
 #pragma unroll
-      for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + jf);
+      for (int c = 0; c < 3; c++) v[c] = ldg(xin + (size_t)c * A.istride + jf);
 #pragma unroll
       for (int e = 0; e < 9; e++) uf[e] = ldlink(ul + (size_t)e * V + out_base + k);
 #pragma unroll
-      for (int c = 0; c < 3; c++) w[c] = ldg(A.xin + (size_t)c * A.istride + jb);
+      for (int c = 0; c < 3; c++) w[c] = ldg(xin + (size_t)c * A.istride + jb);
 #pragma unroll
       for (int e = 0; e < 9; e++) ub[e] = ldlink(ul + (size_t)e * V + in_base + jb);
       double2 t[3], q[3];
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       double2 o = make_double2(A.c * acc[c].x, A.c * acc[c].y);
-      A.out[(size_t)c * A.ostride + k] = o;
+      A.out[(size_t)c * A.ostride + out_off + k] = o;
       if (RED != kRedNone) {
         // Re <xs, out>, xs is the same-site operand (p in CG's A p)
         dot = fma(xsv[c].x, o.x, dot);
@@ -240,13 +247,17 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
   const Geom &g = A.g;
   const int nh = g.nh;
   const size_t V = (size_t)g.V;
-  const size_t in_base = (size_t)(1 - A.po) * nh;
-  const size_t out_base = (size_t)A.po * nh;
+  const int po = A.both ? (int)(blockIdx.x & 1) : A.po;
+  const int block = A.both ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> A.both;
+  const size_t in_base = (size_t)(1 - po) * nh;
+  const size_t out_base = (size_t)po * nh;
+  const size_t in_off = A.both ? in_base : 0, out_off = A.both ? out_base : 0;
+  const double2 *__restrict__ xin = A.xin + in_off;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double dot = 0.0;
   auto gather = [&](int n, double2 v[3]) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) v[c] = ldg(A.xin + (size_t)c * A.istride + n);
+    for (int c = 0; c < 3; c++) v[c] = ldg(xin + (size_t)c * A.istride + n);
     if (CG == 1 && A.cg.it > 0) {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
@@ -255,11 +266,11 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
       }
     }
   };
-  for (int j0 = blockIdx.x * kSplitSites; j0 < A.nsites; j0 += gridDim.x * kSplitSites) {
+  for (int j0 = block * kSplitSites; j0 < A.nsites; j0 += blocks * kSplitSites) {
     const bool on = j0 + lane < A.nsites;
     const int k = out_site(A, on ? j0 + lane : j0);
     int x[4], lex;
-    site_coords(g, A.po, k, x, lex);
+    site_coords(g, po, k, x, lex);
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
       const int n = w * kPer + q, l = n >> 1;  // term n: link l, forward (even n) or backward
@@ -297,7 +308,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
       const int c = w;
       double2 acc = make_double2(0.0, 0.0), xsv = acc;
       if (INIT > 0) {
-        xsv = __ldcg(A.xs + (size_t)c * A.sstride + k);
+        xsv = __ldcg(A.xs + (size_t)c * A.sstride + out_off + k);
         if (CG == 2) {  // xs is r
           double2 *p = A.cg.p + (size_t)c * nh + k;
           if (A.cg.it > 0) {
@@ -309,7 +320,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
         acc = make_double2(A.b * xsv.x, A.b * xsv.y);
       }
       if (INIT == 2) {
-        const double2 rv = __ldcg(A.rin + (size_t)c * A.rstride + k);
+        const double2 rv = __ldcg(A.rin + (size_t)c * A.rstride + out_off + k);
         acc.x = fma(A.a, rv.x, acc.x);
         acc.y = fma(A.a, rv.y, acc.y);
       }
@@ -325,7 +336,7 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
         }
       }
       const double2 o = make_double2(A.c * acc.x, A.c * acc.y);
-      A.out[(size_t)c * A.ostride + k] = o;
+      A.out[(size_t)c * A.ostride + out_off + k] = o;
       if (RED != kRedNone || CG == 2) {
         dot = fma(xsv.x, o.x, dot);
         dot = fma(xsv.y, o.y, dot);
@@ -352,11 +363,12 @@ constexpr int kSplitMax = NL == 8 ? 196608 : 65536;
 
 template <int NL, int HOP, int INIT, int RED>
 static void launch64(const DslashArgs64 &A) {
-  if (A.nsites <= kSplitMax<NL>) {
-    const int grid = std::min((A.nsites + kSplitSites - 1) / kSplitSites, num_sms() * 3);
-    launch_pdl(dslash64_split_kernel<NL, HOP, INIT, RED>, grid, kBlock, A);
+  const int par = A.both ? 2 : 1;  // parities in the launch
+  if (par * A.nsites <= kSplitMax<NL>) {
+    const int grid = std::min((A.nsites + kSplitSites - 1) / kSplitSites, num_sms() * 3 / par);
+    launch_pdl(dslash64_split_kernel<NL, HOP, INIT, RED>, par * grid, kBlock, A);
   } else {
-    launch_pdl(dslash64_kernel<NL, HOP, INIT, RED>, grid_for(A.nsites, kBlock, 6), kBlock, A);
+    launch_pdl(dslash64_kernel<NL, HOP, INIT, RED>, par * grid_for(A.nsites, kBlock, 6 / par), kBlock, A);
   }
   note_launch();
 }
@@ -408,7 +420,37 @@ int dslash64(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, C
   A.k0 = A.k2 = 0;
   A.n1 = A.nsites = g.nh;
   A.rowlen = A.pitch = 0;
+  A.both = 0;
   int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, red) : dispatch64<4>(A, hop, init, red);
+  if (rc) return rc;
+  QS_LAUNCH_CHECK();
+  return QEXSTAG_OK;
+}
+
+// Both half sweeps of the operator on whole-lattice fields (stride V) in one
+// launch: out = c (a rin + b x + (2D) x).  They are independent, and a link
+// that one reads as the forward link of its own site the other reads as the
+// backward link of a site nearby: side by side, the second read finds it in
+// L2, where one launch after the other had the links from HBM twice.  D, us,
+// two launches / one: 12 x 10 x 14 x 18 fat+Naik 18.6 / 17.6, 24^4 147 / 92, 32^4
+// 411 / 386 (three time slices of links, the reach of the long hops, are most
+// of L2 there); naive 24^4 80 / 51.
+int dslash64_both(const qexstag_links_s *gl, double2 *out, const double2 *x, const double2 *rin, double a, double b,
+                  double c, int init) {
+  const Geom &g = gl->l->g;
+  DslashArgs64 A = {};
+  A.g = g;
+  A.u = gl->u64;
+  A.xin = A.xs = x;
+  A.rin = rin;
+  A.out = out;
+  A.istride = A.sstride = A.rstride = A.ostride = g.V;
+  A.a = a;
+  A.b = b;
+  A.c = c;
+  A.n1 = A.nsites = g.nh;
+  A.both = 1;
+  const int rc = gl->nl == 8 ? dispatch64<8>(A, +1, init, kRedNone) : dispatch64<4>(A, +1, init, kRedNone);
   if (rc) return rc;
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;

@@ -122,6 +122,8 @@ int schur64_fused(const qexstag_links_s *gl, int par, const CgFused &F, double m
 int schur64(const qexstag_links_s *g, int par, VecD r, CVecD x, VecD t, double m2,
             int red = kRedNone, void *state = nullptr, const int *done = nullptr,
             double *dot_out = nullptr, const Progress &progress = Progress());
+int dslash64_both(const qexstag_links_s *gl, double2 *out, const double2 *x, const double2 *rin, double a, double b,
+                  double c, int init);
 int dslash64_ranges(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, double b, double c,
                     int hop, int k0, int k1, int k2, int k3, const int *done);
 int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, double b, double c, int hop,

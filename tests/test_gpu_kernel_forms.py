@@ -148,3 +148,29 @@ def test_batch_partitions(cuda, shapes):
         x, ax = S.to_host_vector(x), o.vec()
         o.stagD2ee(ax, x, m * m)
         assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
+
+
+# both parities in one launch, spread over warps (720 even sites) and not (69632
+# naive, 165888 fat+Naik): the same bits as one parity after the other
+@pytest.mark.parametrize("dims,naik", [((4, 6, 6, 10), 0), ((4, 6, 6, 10), 1), ((16, 16, 16, 34), 0),
+                                       ((24, 24, 24, 24), 1)])
+def test_both_parities_in_one_launch(cuda, dims, naik):
+    torch, V = cuda, F.volume(dims)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def field(*shape):
+        return torch.view_as_complex(torch.randn(shape + (2,), dtype=torch.float64, device="cuda", generator=gen))
+
+    s = S.Staggered(S.Layout(dims), field(8 if naik else 4, 3, 3, V))
+    x, r0 = field(3, V), field(3, V)
+    for m, sc, a in ((0.1, 1.0, 0.0), (0.0, -1.0, 0.0), (0.2, 0.5, 0.7)):
+        one, two = r0.clone(), r0.clone()
+        s.stagD(S.L.ALL, one, x, m, sc, a)
+        s.stagD(S.L.EVEN, two, x, m, sc, a)
+        s.stagD(S.L.ODD, two, x, m, sc, a)
+        assert torch.equal(one, two)
+    one, two = x.clone(), x.clone()  # in place: odd sites see the new even ones
+    s.D(one, one, 0.1)
+    s.stagD(S.L.EVEN, two, two, 0.1)
+    s.stagD(S.L.ODD, two, two, 0.1)
+    assert torch.equal(one, two)
