@@ -310,11 +310,11 @@ long long launch_count();
 // launch a kernel that begins with pdl_wait() with programmatic stream
 // serialisation on the library's stream
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl2(void (*kern)(KArgs...), dim3 grid, int block, Args... args) {
+inline cudaError_t launch_pdl2(void (*kern)(KArgs...), dim3 grid, int block, int shared, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = (size_t)shared;
   cfg.stream = stream();
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -325,7 +325,7 @@ inline cudaError_t launch_pdl2(void (*kern)(KArgs...), dim3 grid, int block, Arg
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, Args... args) {
-  return launch_pdl2(kern, dim3((unsigned)grid), block, args...);
+  return launch_pdl2(kern, dim3((unsigned)grid), block, 0, args...);
 }
 
 inline int grid_for(long n, int block = kBlock, int per_sm = 8) {

@@ -101,22 +101,20 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // ---------------------------------------------------------------------------
 // FP32 multi-right-hand-side Dslash on pairs of right-hand sides.  A block is
-// eight warps: a set of 32 sites takes 4 G of them, G = 1 or 2 groups of NP
-// pairs times the four directions, and a block holds 2 / G sets.  Warp
-// (mu, group) forms the direction's hops, forward and backward, fat and long,
-// for its pairs: every link is read from HBM once and from L1 by the other
-// group, a vector load brings both right-hand sides of a pair, and the sums
-// run in FP32x2 arithmetic with the link's parts broadcast.  The four
-// directions' sums meet in shared memory.
+// G = 1, 2 or 4 pairs by S = kBlock / G sites, a thread one pair of one site:
+// a 16-byte vector load brings both right-hand sides, and the sums run in
+// FP32x2 arithmetic with the link's parts broadcast.  Every operand passes
+// through shared memory by asynchronous copies: a stage holds one hop's links
+// of the block's sites, which its pairs share, and each thread's own vectors,
+// and the copies run two or three hops ahead, from one set of sites to the next
+// without a break.
 //
-// Bound by the latency of the gathers through L2 and by how many sites the
-// register file keeps in flight: at 16^4 fat+Naik with 8 right-hand sides 24 us
-// (first sweep) and 32 us (second, with the sums), as a thread that walks all
-// hops of 4 right-hand sides took; one pair a thread in 512-thread blocks took
-// 27 and 39 us at 64 registers, 35 and 47 at 128.
+// Bound by the latency of the gathers through L2: with loads to registers, one
+// hop of 256 sites an SM in flight, a sweep at 16^4 fat+Naik with 8 right-hand
+// sides took 24 us (32 us with the sums), whether a thread walked all hops or
+// the directions were spread over warps; staged, 17 and 25 us.  128-thread
+// blocks with the terms in a loop, more of them on an SM, took 19 and 26 us.
 // ---------------------------------------------------------------------------
-
-constexpr int kMrhsSites = 32;  // sites of a set
 
 struct MrhsArgs {
   Geom g;
@@ -135,6 +133,21 @@ struct MrhsArgs {
   Progress progress;  // posted by this launch (the first half sweep)
 };
 
+template <int G>
+struct MrhsStage {
+  static constexpr int kSites = kBlock / G, kStages = G == 4 ? 4 : G == 2 ? 3 : 2;
+  float4 link[5][kSites];  // 18 reals (the last two in the first half of [4]) or 12
+  float4 vec[G][3][kSites];
+};
+
+__device__ __forceinline__ unsigned shared_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(shared_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy8_async(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(shared_addr(dst)), "l"(src) : "memory");
+}
+
 // (re, im) += (ar, ai) (vr, vi) for both right-hand sides of a pair, nai = -ai
 __device__ __forceinline__ void pair_mac(float2 &re, float2 &im, float ar, float ai, float nai, float2 vr, float2 vi) {
   const float2 ar2 = make_float2(ar, ar), ai2 = make_float2(ai, ai), nai2 = make_float2(nai, nai);
@@ -144,10 +157,12 @@ __device__ __forceinline__ void pair_mac(float2 &re, float2 &im, float ar, float
   im = __ffma2_rn(ai2, vr, im);
 }
 
-template <int NL, int HOP, int INIT, int RED, int R12, int NP, int G>
-__global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A) {
-  constexpr int kSets = 2 / G;
-  __shared__ float4 part[kSets][4][G * NP][3][kMrhsSites];
+template <int NL, int HOP, int INIT, int RED, int R12, int G>
+__global__ void __launch_bounds__(kBlock, 3) dslash_mrhs_kernel(const MrhsArgs A) {
+  constexpr int S = MrhsStage<G>::kSites, kStages = MrhsStage<G>::kStages;
+  constexpr int kTerms = 2 * NL;  // term n: link n / 2, forward (even n) or backward
+  extern __shared__ __align__(16) unsigned char shared_bytes[];
+  MrhsStage<G> *stage = reinterpret_cast<MrhsStage<G> *>(shared_bytes);
   pdl_wait();
   post_progress(A.progress);
   if (A.st->done) return;
@@ -156,84 +171,105 @@ __global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A
   const size_t V = (size_t)g.V;
   const size_t in_base = (size_t)(1 - A.po) * nh;
   const size_t out_base = (size_t)A.po * nh;
-  const int lane_ = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int mu = w & 3, grp = G == 2 ? w >> 2 : 0, set = G == 2 ? 0 : w >> 2;
-  // after the meeting: warp w adds pair fp of set fset
-  const int fset = w / (G * NP), fp = w - fset * (G * NP);
-  const bool adds = fset < kSets && fp < A.npair;
-  double dot[2] = {0.0, 0.0};
-  for (int k0 = blockIdx.x * (kMrhsSites * kSets); k0 < nh; k0 += gridDim.x * (kMrhsSites * kSets)) {
-    {
-      const int kk = k0 + set * kMrhsSites + lane_;
-      const int k = min(kk, nh - 1);
-      int x[4], lex;
-      site_coords(g, A.po, k, x, lex);
-      float2 re[NP][3], im[NP][3];
+  const int pair = threadIdx.x / S, sl = threadIdx.x - pair * S;
+  const bool on = pair < A.npair;  // the other threads copy links only
+  struct Site {
+    int k, lex, x[4];
+  } cur, nxt;
+  auto at = [&](int k0, Site &s) {
+    s.k = min(k0 + sl, nh - 1);
+    site_coords(g, A.po, s.k, s.x, s.lex);
+  };
+  // term n of site s into a stage
+  auto fetch = [&](const Site &s, int n, int slot) {
+    const int l = n >> 1, mu = Hop<NL>::mu(l), len = Hop<NL>::len(l);
+    const bool lng = NL == 8 && (l & 1);
+    const int f = NL == 8 ? (l >> 1) : l;
+    const int jn = nbr_half(g, s.x, s.lex, mu, (n & 1) ? -len : len);
+    const size_t us = (n & 1) ? in_base + jn : out_base + s.k;
+    MrhsStage<G> &st = stage[slot];
+    const int words = lng && R12 ? 3 : 4;
+    const float4 *c = (lng ? A.L.f32_long : A.L.f32_fat) + (size_t)f * words * V + us;
 #pragma unroll
-      for (int q = 0; q < NP; q++)
+    for (int e = 0; e < words; e += G)
+      if (e + pair < words) copy16_async(&st.link[e + pair][sl], c + (size_t)(e + pair) * V);
+    if (words == 4 && pair == 0)
+      copy8_async(&st.link[4][sl], (lng ? A.L.f32_long_tail : A.L.f32_fat_tail) + (size_t)f * V + us);
+    if (on) {
+      const float4 *xp = A.xin + (size_t)pair * A.irs + jn;
 #pragma unroll
-        for (int c = 0; c < 3; c++) re[q][c] = im[q][c] = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int h = 0; h < NL / 4; h++) {
-        const int len = h == 0 ? 1 : 3;
-#pragma unroll
-        for (int dir = 0; dir < 2; dir++) {
-          const int jn = (lex + lex_step(g, x, mu, dir ? -len : len)) >> 1;
-          const size_t us = dir ? in_base + jn : out_base + k;
-          float2 u[9];
-          if (h == 1 && R12)
-            load_long12<kF32>(A.L, mu, us, V, dir ? long_sign_bck(g, x, mu) : long_sign_fwd(g, x, mu), u);
-          else if (h == 1)
-            load_link18<kF32>(A.L.f32_long, A.L.f32_long_tail, nullptr, nullptr, mu, us, V, u);
-          else
-            load_link18<kF32>(A.L.f32_fat, A.L.f32_fat_tail, nullptr, nullptr, mu, us, V, u);
-#pragma unroll
-          for (int q = 0; q < NP; q++) {
-            const int p = grp * NP + q;
-            if (p < A.npair) {
-              const float4 *xp = A.xin + (size_t)p * A.irs + jn;
-              float4 v[3];
-#pragma unroll
-              for (int c = 0; c < 3; c++) v[c] = ldg(xp + (size_t)c * nh);
-#pragma unroll
-              for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                  const float2 vr = make_float2(v[c].x, v[c].y), vi = make_float2(v[c].z, v[c].w);
-                  // forward + U_ic v_c; backward - conj(U_ci) v_c
-                  if (dir == 0)
-                    pair_mac(re[q][i], im[q][i], u[3 * i + c].x, u[3 * i + c].y, -u[3 * i + c].y, vr, vi);
-                  else
-                    pair_mac(re[q][i], im[q][i], -u[3 * c + i].x, u[3 * c + i].y, -u[3 * c + i].y, vr, vi);
-                }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < NP; q++)
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          part[set][mu][grp * NP + q][c][lane_] = make_float4(re[q][c].x, re[q][c].y, im[q][c].x, im[q][c].y);
+      for (int i = 0; i < 3; i++) copy16_async(&st.vec[pair][i][sl], xp + (size_t)i * nh);
     }
-    __syncthreads();
-    const int k = k0 + fset * kMrhsSites + lane_;
-    if (adds && k < nh) {
+  };
+  const int step = gridDim.x * S;
+  int slot = 0;  // of the term being summed
+  at(blockIdx.x * S, cur);
+#pragma unroll
+  for (int n = 0; n < kStages - 1; n++) {
+    fetch(cur, n, n);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  double dot[2] = {0.0, 0.0};
+  for (int k0 = blockIdx.x * S; k0 < nh; k0 += step) {
+    const bool more = k0 + step < nh;
+    if (more) at(k0 + step, nxt);
+    float2 re[3], im[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) re[c] = im[c] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int n = 0; n < kTerms; n++) {
+      const int l = n >> 1, mu = Hop<NL>::mu(l);
+      const bool lng = NL == 8 && (l & 1);
+      asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");  // this thread's copies of term n
+      __syncthreads();  // everyone's; and the term before has been read
+      {
+        const int ahead = n + kStages - 1;
+        int to = slot + kStages - 1;
+        if (to >= kStages) to -= kStages;
+        if (ahead < kTerms)
+          fetch(cur, ahead, to);
+        else if (more)
+          fetch(nxt, ahead - kTerms, to);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+      const MrhsStage<G> &st = stage[slot];
+      if (++slot == kStages) slot = 0;
+      if (on) {
+        float2 u[9];
+#pragma unroll
+        for (int e = 0; e < (lng && R12 ? 3 : 4); e++) {
+          const float4 q = st.link[e][sl];
+          u[2 * e] = make_float2(q.x, q.y);
+          u[2 * e + 1] = make_float2(q.z, q.w);
+        }
+        if (lng && R12)
+          recon_row2(u, ((n & 1) ? long_sign_bck(g, cur.x, mu) : long_sign_fwd(g, cur.x, mu)) * A.L.long_rc);
+        else
+          u[8] = *reinterpret_cast<const float2 *>(&st.link[4][sl]);
+        float4 v[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = st.vec[pair][c][sl];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            const float2 vr = make_float2(v[c].x, v[c].y), vi = make_float2(v[c].z, v[c].w);
+            // forward + U_ic v_c; backward - conj(U_ci) v_c
+            if ((n & 1) == 0)
+              pair_mac(re[i], im[i], u[3 * i + c].x, u[3 * i + c].y, -u[3 * i + c].y, vr, vi);
+            else
+              pair_mac(re[i], im[i], -u[3 * c + i].x, u[3 * c + i].y, -u[3 * c + i].y, vr, vi);
+          }
+      }
+    }
+    if (on && k0 + sl < nh) {
       float d0 = 0.f, d1 = 0.f;
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-          const float4 t = part[fset][m][fp][c][lane_];
-          o.x += t.x;
-          o.y += t.y;
-          o.z += t.z;
-          o.w += t.w;
-        }
+        float4 o = make_float4(re[c].x, re[c].y, im[c].x, im[c].y);
         if (HOP < 0) o = make_float4(-o.x, -o.y, -o.z, -o.w);
         if (INIT) {
-          const float4 s = __ldcg(A.xs + (size_t)fp * A.srs + (size_t)c * nh + k);
+          const float4 s = __ldcg(A.xs + (size_t)pair * A.srs + (size_t)c * nh + cur.k);
           o.x = fmaf(A.b, s.x, o.x);
           o.y = fmaf(A.b, s.y, o.y);
           o.z = fmaf(A.b, s.z, o.z);
@@ -243,34 +279,41 @@ __global__ void __launch_bounds__(kBlock, 2) dslash_mrhs_kernel(const MrhsArgs A
             d1 = fmaf(s.y, o.y, fmaf(s.w, o.w, d1));
           }
         }
-        A.out[(size_t)fp * A.ors + (size_t)c * nh + k] = o;
+        A.out[(size_t)pair * A.ors + (size_t)c * nh + cur.k] = o;
       }
       if (RED) {
         dot[0] += (double)d0;
         dot[1] += (double)d1;
       }
     }
-    __syncthreads();
+    cur = nxt;
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (RED) {
-    const int stride = gridDim.x * kSets;
+    // a slot per warp and right-hand side; a warp holds one pair
+    const int stride = gridDim.x * (S / 32), slot_ = blockIdx.x * (S / 32) + sl / 32;
     dot[0] = warp_sum(dot[0]);
     dot[1] = warp_sum(dot[1]);
-    if (adds && lane_ == 0) {
-      const int slot = blockIdx.x * kSets + fset;
-      A.partials[(size_t)(2 * fp) * stride + slot] = dot[0];
-      if (2 * fp + 1 < A.nr) A.partials[(size_t)(2 * fp + 1) * stride + slot] = dot[1];
+    if (on && (threadIdx.x & 31) == 0) {
+      A.partials[(size_t)(2 * pair) * stride + slot_] = dot[0];
+      if (2 * pair + 1 < A.nr) A.partials[(size_t)(2 * pair + 1) * stride + slot_] = dot[1];
     }
-    double s;
-    if (rhs_reduce(A.nr, A.partials, stride, A.ticket, gridDim.x, s) && w < A.nr && lane_ == 0) A.wst->pAp[w] = s;
+    const int w = threadIdx.x >> 5;
+    double t;
+    if (rhs_reduce(A.nr, A.partials, stride, A.ticket, gridDim.x, t) && w < A.nr && (threadIdx.x & 31) == 0)
+      A.wst->pAp[w] = t;
   }
 }
 
-template <int NL, int R12, int NP, int G>
-static void mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
-  const int sets = 2 / G, per = kMrhsSites * sets;
-  // slots of the reduction: 8 right-hand sides share red_partials
-  const int grid = std::min({(A.nh + per - 1) / per, num_sms() * 6, kMaxRedBlocks / sets});
+template <int NL, int R12, int G>
+static int mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
+  constexpr int S = MrhsStage<G>::kSites, bytes = (int)sizeof(MrhsStage<G>) * MrhsStage<G>::kStages;
+  auto *first = dslash_mrhs_kernel<NL, 1, 0, 0, R12, G>;
+  auto *second = dslash_mrhs_kernel<NL, -1, 1, 1, R12, G>;
+  QS_CUDA(cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  QS_CUDA(cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  // one wave of three blocks per SM; kMaxRedBlocks reduction slots per right-hand side
+  const int grid = std::min({(A.nh + S - 1) / S, num_sms() * 3, kMaxRedBlocks / (S / 32)});
   const size_t vs = (size_t)3 * A.nh;
   A.po = 1 - par;
   A.xin = p;
@@ -280,7 +323,7 @@ static void mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *
   A.out = t;
   A.ors = vs;
   A.b = 0.f;
-  launch_pdl(dslash_mrhs_kernel<NL, 1, 0, 0, R12, NP, G>, grid, kBlock, A);
+  launch_pdl2(first, dim3(grid), kBlock, bytes, A);
   A.progress = Progress();
   A.po = par;
   A.xin = t;
@@ -290,18 +333,17 @@ static void mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *
   A.out = ap;
   A.ors = vs;
   A.b = b4m2;
-  launch_pdl(dslash_mrhs_kernel<NL, -1, 1, 1, R12, NP, G>, grid, kBlock, A);
+  launch_pdl2(second, dim3(grid), kBlock, bytes, A);
   note_launch(2);
+  QS_LAUNCH_CHECK();
+  return QEXSTAG_OK;
 }
 
 template <int NL, int R12>
-static void mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
-  if (A.npair == 1)
-    mrhs_pair<NL, R12, 1, 1>(A, par, p, prs, t, ap, b4m2);
-  else if (A.npair == 2)
-    mrhs_pair<NL, R12, 2, 1>(A, par, p, prs, t, ap, b4m2);
-  else
-    mrhs_pair<NL, R12, 2, 2>(A, par, p, prs, t, ap, b4m2);
+static int mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
+  if (A.npair == 1) return mrhs_pair<NL, R12, 1>(A, par, p, prs, t, ap, b4m2);
+  if (A.npair == 2) return mrhs_pair<NL, R12, 2>(A, par, p, prs, t, ap, b4m2);
+  return mrhs_pair<NL, R12, 4>(A, par, p, prs, t, ap, b4m2);
 }
 
 // pair j of p at p + j*prs; of t and ap at j*3*nh
@@ -320,16 +362,8 @@ static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p
   A.ticket = red_tickets();
   A.progress = progress;
   const float b4 = (float)(4.0 * m2);
-  if (g->nl == 8) {
-    if (g->low.recon12)
-      mrhs_pairs<8, 1>(A, par, p, prs, t, ap, b4);
-    else
-      mrhs_pairs<8, 0>(A, par, p, prs, t, ap, b4);
-  } else {
-    mrhs_pairs<4, 0>(A, par, p, prs, t, ap, b4);
-  }
-  QS_LAUNCH_CHECK();
-  return QEXSTAG_OK;
+  if (g->nl == 4) return mrhs_pairs<4, 0>(A, par, p, prs, t, ap, b4);
+  return g->low.recon12 ? mrhs_pairs<8, 1>(A, par, p, prs, t, ap, b4) : mrhs_pairs<8, 0>(A, par, p, prs, t, ap, b4);
 }
 
 // ---------------------------------------------------------------------------
@@ -673,8 +707,8 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
       if (seen & kPaceStop) break;
       if ((rc2 = schur(v))) return rc2;
       pace.queued++;
-      launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, v, st, red_partials(), red_tickets());
-      launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, v, (const CgmState *)st, (int)pace.queued);
+      launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, 0, v, st, red_partials(), red_tickets());
+      launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, 0, v, (const CgmState *)st, (int)pace.queued);
       note_launch(2);
       QS_LAUNCH_CHECK();
     }
