@@ -5,11 +5,11 @@
 // QEX tiles 16 sites x 8 vectors so that a site's links are loaded once for
 // all vectors.  Here a block of 256 threads is G warp-uniform groups of
 // 256/G sites (G = 1, 2 or 4); group q applies the operator to vectors
-// 2q and 2q+1 of its sites.  Every group reads the same links, so each link
-// comes from HBM once per site and from L1 for the other groups, and every
-// vector's loads stay coalesced across the warp.  Up to 8 vectors per
-// launch.  Accumulation follows stagDPN: the mass term, then the forward
-// hops, then the backward hops.
+// 2q and 2q+1 of its sites.  Every group uses the same links, which come from
+// HBM once per site: from L1 for the other groups, or through shared memory
+// (the kernel with the ring, below).  Every vector's loads stay coalesced
+// across the warp.  Up to 8 vectors per launch.  Accumulation follows stagDPN:
+// the mass term, then the forward hops, then the backward hops.
 //
 // Compulsory bytes per output site: links (nlinks x 2 x 144 B: a forward
 // link at the site and a backward link at the neighbour) + n x (48 B own
@@ -121,6 +121,146 @@ __global__ void __launch_bounds__(kBlock, 2) dslashN64_kernel(const DnArgs A) {
   }
 }
 
+// The same sums in the same order with more sites in flight.  The kernel above
+// is bound by latency: its links and unrolled hops take the register file with
+// 16 warps an SM.  Here the links of kDnAhead further terms are on their way to
+// a ring in shared memory, which takes them out of the registers, and the terms
+// run in a loop: 80 registers, 24 warps.  A block has one set of sites, and the
+// blocks start in order, so that a hop's neighbours are still in L2 (six blocks
+// an SM in strides over the sites: 340 us below).  24^3 x 48, fat+Naik, 8
+// vectors: 388 -> 319 us, of 172 us for the compulsory bytes at 6.65 TB/s; what
+// is left is the vectors' gathers.  The vectors in the ring as well took 360 us,
+// their loads one term ahead in registers 382 us, the directions spread over
+// warps 753 us.
+template <int G>
+constexpr int kDnAhead = G == 4 ? 3 : 1;  // what the 48 KB of a block hold
+
+__device__ __forceinline__ void copy_link_async(double2 *dst, const double2 *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+template <int NL, int G>
+__global__ void __launch_bounds__(kBlock, 3) dslashN64_ring_kernel(const DnArgs A) {
+  constexpr int S = kBlock / G;       // sites per block step
+  constexpr int kTerms = 2 * NL;      // forward hops, then backward ones
+  constexpr int kRing = kDnAhead<G> + 1;
+  __shared__ double2 ring[kRing][9][S];
+  const Geom &g = A.g;
+  const int nh = g.nh;
+  const size_t V = (size_t)g.V;
+  const int grp = threadIdx.x / S, sl = threadIdx.x - grp * S;
+  const int j0 = grp * kDnPer;
+  const int nq = min(kDnPer, A.n - j0);  // may be <= 0: such a group copies links only
+  const size_t in_base = (size_t)(1 - A.po) * nh, out_base = (size_t)A.po * nh;
+  const int kk = blockIdx.x * S + sl, k = min(kk, nh - 1);
+  int x[4], lex;
+  site_coords(g, A.po, k, x, lex);
+  auto nbr = [&](int n) {
+    const int l = n < NL ? n : n - NL, len = Hop<NL>::len(l);
+    return (lex + lex_step(g, x, Hop<NL>::mu(l), n < NL ? len : -len)) >> 1;
+  };
+  auto fetch = [&](int n) {
+    if (n < kTerms) {
+      const int l = n < NL ? n : n - NL;
+      const double2 *ul = A.u + (size_t)l * 9 * V + (n < NL ? out_base + k : in_base + nbr(n));
+#pragma unroll
+      for (int e = 0; e < 9; e += G)
+        if (e + grp < 9) copy_link_async(&ring[n % kRing][e + grp][sl], ul + (size_t)(e + grp) * V);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int n = 0; n < kDnAhead<G>; n++) fetch(n);
+  double2 acc[kDnPer][3];
+#pragma unroll
+  for (int q = 0; q < kDnPer; q++) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double2 v = make_double2(0.0, 0.0);
+      if (q < nq) v = ldg(A.x[j0 + q] + (size_t)c * A.xstride + out_base + k);
+      acc[q][c] = make_double2(A.m * v.x, A.m * v.y);
+    }
+  }
+#pragma unroll 1
+  for (int n = 0; n < kTerms; n++) {
+    double2 v[kDnPer][3];
+    const int jn = nbr(n);
+#pragma unroll
+    for (int q = 0; q < kDnPer; q++)
+      if (q < nq) {
+        const double2 *xq = A.x[j0 + q] + in_base + jn;
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[q][c] = ldg(xq + (size_t)c * A.xstride);
+      }
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDnAhead<G> - 1) : "memory");  // this thread's copies of term n
+    __syncthreads();  // everyone's; and term n - 1's links have been read
+    fetch(n + kDnAhead<G>);
+    const int slot = n % kRing;
+    if (n < NL) {  // forward: + U_l(s) x(s + d_l)
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double2 u = ring[slot][3 * i + c][sl];
+#pragma unroll
+          for (int q = 0; q < kDnPer; q++)
+            if (q < nq) acc[q][i] = cmadd(acc[q][i], u, v[q][c]);
+        }
+    } else {  // backward: - U_l(s - d_l)^dagger x(s - d_l)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double2 t[kDnPer];
+#pragma unroll
+        for (int q = 0; q < kDnPer; q++) t[q] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double2 u = ring[slot][3 * c + i][sl];
+#pragma unroll
+          for (int q = 0; q < kDnPer; q++)
+            if (q < nq) t[q] = cjmadd(t[q], u, v[q][c]);
+        }
+#pragma unroll
+        for (int q = 0; q < kDnPer; q++) {
+          acc[q][i].x -= t[q].x;
+          acc[q][i].y -= t[q].y;
+        }
+      }
+    }
+  }
+  if (kk < nh) {
+#pragma unroll
+    for (int q = 0; q < kDnPer; q++) {
+      if (q < nq) {
+        double2 *rq = A.r[j0 + q] + out_base + k;
+#pragma unroll
+        for (int c = 0; c < 3; c++) rq[(size_t)c * A.rstride] = acc[q][c];
+      }
+    }
+  }
+}
+
+// The ring pays from about 260000 sites times vectors on; below, its barriers
+// cost more than its warps give.  us, first kernel / ring, fat+Naik: 16^4 (32768
+// sites a parity) 8 vectors 42 / 44; 20^4 3 vectors 50 / 52, 4 60 / 54, 8 102 /
+// 87; 24^4 3 vectors 95 / 89, 8 198 / 171; 32^4 3 vectors 411 / 300, 8 608 / 589;
+// naive 16^4 8 vectors 25 / 25, 20^4 3 29 / 30, 4 33 / 32, 32^4 8 353 / 304.  One
+// group, two vectors at most, has no use for it: 32^4 190 / 313.
+constexpr long kDnRingFrom = 262144;
+
+template <int NL>
+static void launch_dn(const DnArgs &A) {
+  const long nh = A.g.nh;
+  const int S = kBlock / A.groups;
+  const int sets = (int)((nh + S - 1) / S);
+  if (A.groups == 1 || nh * A.n <= kDnRingFrom)
+    dslashN64_kernel<NL><<<std::min(sets, num_sms() * 4), kBlock, 0, stream()>>>(A);
+  else if (A.groups == 2)
+    dslashN64_ring_kernel<NL, 2><<<sets, kBlock, 0, stream()>>>(A);
+  else
+    dslashN64_ring_kernel<NL, 4><<<sets, kBlock, 0, stream()>>>(A);
+}
+
 // r[i] (parity po) = m x[i] + (2D) x[i] for i < n; full-lattice device
 // fields with strides xstride, rstride.  Vectors go 8 to a launch.
 int dslashN64(const qexstag_links_s *gl, int po, int n, double2 *const *r, int rstride, const double2 *const *x,
@@ -140,12 +280,10 @@ int dslashN64(const qexstag_links_s *gl, int po, int n, double2 *const *r, int r
     }
     A.xstride = xstride;
     A.rstride = rstride;
-    const int S = kBlock / A.groups;
-    const int grid = (int)std::min<long>(((long)g.nh + S - 1) / S, (long)num_sms() * 4);
     if (gl->nl == 8)
-      dslashN64_kernel<8><<<grid, kBlock, 0, stream()>>>(A);
+      launch_dn<8>(A);
     else
-      dslashN64_kernel<4><<<grid, kBlock, 0, stream()>>>(A);
+      launch_dn<4>(A);
     note_launch();
     QS_LAUNCH_CHECK();
   }
