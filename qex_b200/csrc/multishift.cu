@@ -112,9 +112,16 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Bound by the latency of the gathers through L2: with loads to registers, one
 // hop of 256 sites an SM in flight, a sweep at 16^4 fat+Naik with 8 right-hand
 // sides took 24 us (32 us with the sums), whether a thread walked all hops or
-// the directions were spread over warps; staged, 17 and 25 us.  128-thread
-// blocks with the terms in a loop, more of them on an SM, took 19 and 26 us.
+// the directions were spread over warps; staged, 17 and 25 us, and 18 us for the
+// second since cgm_update1 adds its blocks' sums (a last block that added them
+// took 7 us).  Not faster: 128-thread blocks with the terms in a loop (19 us),
+// four blocks an SM with three stages (18 and 20 us), a grid that gives every
+// block as many sets (19 and 20 us).
 // ---------------------------------------------------------------------------
+
+// red_partials is shared by two sums: <p, Ap> from its start, |r|^2 behind it,
+// kCgmSums doubles each over the right-hand sides
+constexpr int kCgmSums = kMaxRedBlocks * 4;
 
 struct MrhsArgs {
   Geom g;
@@ -127,9 +134,7 @@ struct MrhsArgs {
   int nh;
   float b;
   const CgmState *st;
-  CgmState *wst;
   double *partials;
-  unsigned *ticket;
   Progress progress;  // posted by this launch (the first half sweep)
 };
 
@@ -290,7 +295,8 @@ __global__ void __launch_bounds__(kBlock, 3) dslash_mrhs_kernel(const MrhsArgs A
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (RED) {
-    // a slot per warp and right-hand side; a warp holds one pair
+    // <xs, out>: a slot per warp and right-hand side (a warp holds one pair),
+    // which the update's blocks add
     const int stride = gridDim.x * (S / 32), slot_ = blockIdx.x * (S / 32) + sl / 32;
     dot[0] = warp_sum(dot[0]);
     dot[1] = warp_sum(dot[1]);
@@ -298,22 +304,19 @@ __global__ void __launch_bounds__(kBlock, 3) dslash_mrhs_kernel(const MrhsArgs A
       A.partials[(size_t)(2 * pair) * stride + slot_] = dot[0];
       if (2 * pair + 1 < A.nr) A.partials[(size_t)(2 * pair + 1) * stride + slot_] = dot[1];
     }
-    const int w = threadIdx.x >> 5;
-    double t;
-    if (rhs_reduce(A.nr, A.partials, stride, A.ticket, gridDim.x, t) && w < A.nr && (threadIdx.x & 31) == 0)
-      A.wst->pAp[w] = t;
   }
 }
 
 template <int NL, int R12, int G>
-static int mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
+static int mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2, int *np) {
   constexpr int S = MrhsStage<G>::kSites, bytes = (int)sizeof(MrhsStage<G>) * MrhsStage<G>::kStages;
   auto *first = dslash_mrhs_kernel<NL, 1, 0, 0, R12, G>;
   auto *second = dslash_mrhs_kernel<NL, -1, 1, 1, R12, G>;
   QS_CUDA(cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   QS_CUDA(cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  // one wave of three blocks per SM; kMaxRedBlocks reduction slots per right-hand side
-  const int grid = std::min({(A.nh + S - 1) / S, num_sms() * 3, kMaxRedBlocks / (S / 32)});
+  // one wave of three blocks per SM; kCgmSums / nr partials per right-hand side
+  const int grid = std::min({(A.nh + S - 1) / S, num_sms() * 3, kCgmSums / A.nr / (S / 32)});
+  *np = grid * (S / 32);
   const size_t vs = (size_t)3 * A.nh;
   A.po = 1 - par;
   A.xin = p;
@@ -340,15 +343,17 @@ static int mrhs_pair(MrhsArgs A, int par, const float4 *p, size_t prs, float4 *t
 }
 
 template <int NL, int R12>
-static int mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2) {
-  if (A.npair == 1) return mrhs_pair<NL, R12, 1>(A, par, p, prs, t, ap, b4m2);
-  if (A.npair == 2) return mrhs_pair<NL, R12, 2>(A, par, p, prs, t, ap, b4m2);
-  return mrhs_pair<NL, R12, 4>(A, par, p, prs, t, ap, b4m2);
+static int mrhs_pairs(const MrhsArgs &A, int par, const float4 *p, size_t prs, float4 *t, float4 *ap, float b4m2,
+                      int *np) {
+  if (A.npair == 1) return mrhs_pair<NL, R12, 1>(A, par, p, prs, t, ap, b4m2, np);
+  if (A.npair == 2) return mrhs_pair<NL, R12, 2>(A, par, p, prs, t, ap, b4m2, np);
+  return mrhs_pair<NL, R12, 4>(A, par, p, prs, t, ap, b4m2, np);
 }
 
-// pair j of p at p + j*prs; of t and ap at j*3*nh
+// pair j of p at p + j*prs; of t and ap at j*3*nh.  *np: partials of <p, Ap>
+// that each right-hand side has in red_partials
 static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p, size_t prs, float4 *t,
-                      float4 *ap, double m2, CgmState *st, const Progress &progress) {
+                      float4 *ap, double m2, CgmState *st, const Progress &progress, int *np) {
   const Geom &geo = g->l->g;
   MrhsArgs A;
   A.g = geo;
@@ -357,13 +362,12 @@ static int schur_mrhs(const qexstag_links_s *g, int par, int nr, const float4 *p
   A.L = lo_links(g->low, kF32);
   A.nh = geo.nh;
   A.st = st;
-  A.wst = st;
   A.partials = red_partials();
-  A.ticket = red_tickets();
   A.progress = progress;
   const float b4 = (float)(4.0 * m2);
-  if (g->nl == 4) return mrhs_pairs<4, 0>(A, par, p, prs, t, ap, b4);
-  return g->low.recon12 ? mrhs_pairs<8, 1>(A, par, p, prs, t, ap, b4) : mrhs_pairs<8, 0>(A, par, p, prs, t, ap, b4);
+  if (g->nl == 4) return mrhs_pairs<4, 0>(A, par, p, prs, t, ap, b4, np);
+  return g->low.recon12 ? mrhs_pairs<8, 1>(A, par, p, prs, t, ap, b4, np)
+                        : mrhs_pairs<8, 0>(A, par, p, prs, t, ap, b4, np);
 }
 
 // ---------------------------------------------------------------------------
@@ -380,26 +384,45 @@ __device__ __forceinline__ void axpy2(L1 &&y, double a, L2 &&x) {
 
 // cgm.nim:157-184 for shift 0: r -= alpha Ap; x0 += alpha p0; |r|^2; then, in
 // the last block, the zeta recurrences of every other shift (cgm.nim:187-200):
-// warp j, lane k for shift k of right-hand side j.  alpha = r2 / <p, Ap> comes
-// from the sums the operator left.  (One thread that walked the 8 x 6 scalars
+// warp j, lane k for shift k of right-hand side j.  alpha = r2 / <p, Ap>: with
+// np > 0 every block adds the np partials that the operator left for its own
+// right-hand sides at pap.  (One thread that walked the 8 x 6 scalars
 // one by one, and two one-thread kernels around it for alpha and the end
 // test, took 25 us an iteration at 16^4; this takes 11.5.  Whole 8-system,
 // 6-shift solve: 238 -> 181 ms.)
 template <class VT>
-__global__ void __launch_bounds__(kBlock) cgm_update1_kernel(CgmVecs<VT> v, CgmState *st, double *partials,
-                                                            unsigned *ticket) {
+__global__ void __launch_bounds__(kBlock) cgm_update1_kernel(CgmVecs<VT> v, CgmState *st, const double *pap, int np,
+                                                            double *partials, unsigned *ticket) {
   pdl_wait();
   if (st->done) return;
   constexpr int n = Lanes<VT>::n;
   const int nh = v.nh, e = blockIdx.y;
-  __shared__ double sh[n * 32];
+  __shared__ double sh[n * 32], sh_pap[n];
   double a[n], s[n];
   bool any = false;
+  if (np > 0) {
+    double t[n];
+#pragma unroll
+    for (int q = 0; q < n; q++) {
+      t[q] = 0.0;
+      if (e * n + q < st->nrhs)
+        for (int i = threadIdx.x; i < np; i += blockDim.x) t[q] += __ldcg(pap + (size_t)(e * n + q) * np + i);
+    }
+    block_sum<n>(t, sh);
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < n; q++) {
+        sh_pap[q] = t[q];
+        if (blockIdx.x == 0 && e * n + q < st->nrhs) st->pAp[e * n + q] = t[q];  // for the last block
+      }
+    }
+    __syncthreads();
+  }
 #pragma unroll
   for (int q = 0; q < n; q++) {
     const int j = e * n + q;
     const bool on = j < st->nrhs && st->live[j] != 0;
-    const double pAp = on ? st->pAp[j] : 0.0;
+    const double pAp = !on ? 0.0 : np > 0 ? sh_pap[q] : st->pAp[j];
     a[q] = pAp != 0.0 ? st->r2i[j] / pAp : 0.0;
     s[q] = 0.0;
     any |= on;
@@ -447,7 +470,7 @@ __global__ void __launch_bounds__(kBlock) cgm_update1_kernel(CgmVecs<VT> v, CgmS
   int cont = 0;
   if (j < nrhs) {
     const bool live = st->live[j] != 0;
-    const double pAp = st->pAp[j], r2i = st->r2i[j];
+    const double pAp = __ldcg(&st->pAp[j]), r2i = st->r2i[j];
     const double alpha = pAp != 0.0 ? r2i / pAp : 0.0;
     const double beta = r2i != 0.0 ? r2ip1 / r2i : 0.0;
     cont = live && itn < st->maxits && r2ip1 > st->r2stop[j];
@@ -685,14 +708,15 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
   QS_CUDA(cudaMemcpyAsync(st, pin, sizeof(hs), cudaMemcpyHostToDevice, stream()));
   QS_CUDA(cudaMemcpyAsync(pb, (char *)pin + sizeof(hs), sizeof(double2 *) * nrhs, cudaMemcpyHostToDevice,
                           stream()));
-  // grid rows share the GPU; kMaxRedBlocks slots per right-hand side
-  const dim3 grid(std::min(grid_for(nh, kBlock, std::max(1, 8 / nvec)), kMaxRedBlocks), nvec);
+  // grid rows share the GPU; kCgmSums / kMaxRhs slots per right-hand side
+  const dim3 grid(std::min(grid_for(nh, kBlock, std::max(1, 8 / nvec)), kCgmSums / kMaxRhs), nvec);
   Pace pace;
   if ((rc = pace.start(ws, nh))) return rc;
   Progress progress;
   progress.word = pace.word;
   progress.itn = &st->itn;
   progress.stop = &st->done;
+  int np = 0;  // <p, Ap> partials of the pair operator; the others finish the sum
   // an iteration: the operator's two half sweeps and the two updates
   auto solve = [&](auto v, auto schur) -> int {
     using VT = std::remove_pointer_t<decltype(v.r)>;
@@ -707,7 +731,8 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
       if (seen & kPaceStop) break;
       if ((rc2 = schur(v))) return rc2;
       pace.queued++;
-      launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, 0, v, st, red_partials(), red_tickets());
+      launch_pdl2(cgm_update1_kernel<VT>, grid, kBlock, 0, v, st, (const double *)red_partials(), np,
+                  red_partials() + kCgmSums, red_tickets());
       launch_pdl2(cgm_update2_kernel<VT>, grid, kBlock, 0, v, (const CgmState *)st, (int)pace.queued);
       note_launch(2);
       QS_LAUNCH_CHECK();
@@ -726,7 +751,9 @@ static int cgm_core(qexstag_links_s *g, int par, double m2, int nshift, const do
   if (pairs) {
     CgmVecs<float4> v{(float4 *)pr, (float4 *)pap, (float4 *)pt, (float4 *)px, (float4 *)pp, nh, nshift, nvec};
     // p_0 of pair j lives at xs_off(j, 0)
-    rc = solve(v, [&](auto &w) { return schur_mrhs(g, par, nrhs, w.p, w.xs_off(1, 0), w.t, w.ap, m2, st, progress); });
+    rc = solve(v, [&](auto &w) {
+      return schur_mrhs(g, par, nrhs, w.p, w.xs_off(1, 0), w.t, w.ap, m2, st, progress, &np);
+    });
   } else if (fp32) {
     CgmVecs<float2> v{(float2 *)pr, (float2 *)pap, (float2 *)pt, (float2 *)px, (float2 *)pp, nh, nshift, 1};
     rc = solve(v, [&](auto &w) { return schur_lo_v32(g, lprec, par, w.ap, w.p, w.t, m2, &st->pAp[0], progress); });
