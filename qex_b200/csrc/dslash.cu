@@ -44,9 +44,8 @@ struct DslashArgs64 {
   // instead nsites / rowlen runs of rowlen sites, pitch apart, from k0
   int k0, n1, k2, nsites;
   int rowlen, pitch;
-  // both parities in one launch, even blocks on even sites: po is unused and
-  // the fields' pointers are those of the whole lattice
-  int both;
+  // both parities in one launch (BOTH): even blocks on even sites; po is unused
+  // and the fields' pointers are those of the whole lattice
   Progress progress;  // posted by this launch (a solve's first half sweep)
   CgFused cg;         // fused CG (CG > 0)
 };
@@ -116,19 +115,29 @@ __device__ __forceinline__ void reduce_pap(const DslashArgs64 &A, double dot) {
   }
 }
 
-template <int NL, int HOP, int INIT, int RED>
-__global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) {
+// RESIDENT blocks per SM.  Without that bound the compiler stops at 72 to 90
+// registers and waits for each hop's loads before it starts the next hop's; with
+// 128 (two blocks) or 255 (one) it has the loads of several hops in flight, which
+// is worth more than the warps it costs.  us, 72-90 registers / 128 / 255: Schur
+// fat+Naik 32^4 423 / 374 / 380, 24^4 146 / 121 / 121, 16^4 64 / 29 / 26.5; naive
+// 32^4 224 / 190 / 196, 24^4 79 / 62 / 66; D fat+Naik 32^4 361 / 289 / 291, naive
+// 208 / 141 / 145; an FP64 CG iteration at 32^4 fat+Naik 534 / 424 / 427, naive 286
+// / 241 / 247.  At 32^4 fat+Naik the Schur operator moves its compulsory bytes at
+// 6.8 TB/s, above the copy rate: part of the links is still in L2 from the other
+// sweep.  A block for every 256 sites instead of six per SM: 379.
+template <int NL, int HOP, int INIT, int RED, int BOTH, int RESIDENT>
+__global__ void __launch_bounds__(kBlock, RESIDENT) dslash64_kernel(const DslashArgs64 A) {
   pdl_wait();
   post_progress(A.progress);
   if (A.done != nullptr && *A.done) return;
   const Geom &g = A.g;
   const int nh = g.nh;
   const size_t V = (size_t)g.V;
-  const int po = A.both ? (int)(blockIdx.x & 1) : A.po;
-  const int block = A.both ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> A.both;
+  const int po = BOTH ? (int)(blockIdx.x & 1) : A.po;
+  const int block = BOTH ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> BOTH;
   const size_t in_base = (size_t)(1 - po) * nh;
   const size_t out_base = (size_t)po * nh;
-  const size_t in_off = A.both ? in_base : 0, out_off = A.both ? out_base : 0;
+  const size_t in_off = BOTH ? in_base : 0, out_off = BOTH ? out_base : 0;
   const double2 *__restrict__ xin = A.xin + in_off;
   double dot = 0.0;
   for (int j = block * blockDim.x + threadIdx.x; j < A.nsites; j += blocks * blockDim.x) {
@@ -217,19 +226,19 @@ __global__ void __launch_bounds__(kBlock) dslash64_kernel(const DslashArgs64 A) 
 // sum are those of dslash64_kernel, so the result is the same bit for bit.
 //
 // Where the whole-site kernel has too few blocks to fill the GPU, its time
-// is one thread's walk through 8 or 16 dependent rounds of loads; this form
-// takes one or two rounds.  Schur operator (two sweeps), us, whole-site form
-// against this one: 8^4 naive 13.3 / 8.3, 8^3 x 16 fat+Naik 45.5 / 9.6, 16^4
-// fat+Naik 64.6 / 35.2.  With the GPU full it loses to the meeting in shared
-// memory (32^4 fat+Naik 426 / 446).
+// is one thread's walk through 8 or 16 rounds of loads; this form takes one or
+// two rounds.  With the GPU full it loses to the meeting in shared memory.  The
+// figures are at kSplitMax.  At most 128 registers, for the same reason as above
+// (12 x 10 x 14 x 18 fat+Naik: 22.4 us without the bound, 15.4); the sweeps of
+// the fused CG (CG > 0) are faster without it (12^4 18 us an iteration, 21.6).
 constexpr int kSplitSites = 32;
 constexpr int kSplitWarps = kBlock / 32;
 
 // CG > 0: the sweeps of a fused CG iteration.  CG = 1, the first, forms its
 // input r + beta p at the neighbours; CG = 2, the second, forms p at its own
 // sites and leaves each block's part of <p, Ap>.
-template <int NL, int HOP, int INIT, int RED, int CG = 0>
-__global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs64 A) {
+template <int NL, int HOP, int INIT, int RED, int CG = 0, int BOTH = 0>
+__global__ void __launch_bounds__(kBlock, CG ? 0 : 2) dslash64_split_kernel(const DslashArgs64 A) {
   constexpr int kTerms = 2 * NL, kPer = kTerms / kSplitWarps;
   __shared__ double2 term[kTerms][3][kSplitSites];
   pdl_wait();
@@ -247,11 +256,11 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
   const Geom &g = A.g;
   const int nh = g.nh;
   const size_t V = (size_t)g.V;
-  const int po = A.both ? (int)(blockIdx.x & 1) : A.po;
-  const int block = A.both ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> A.both;
+  const int po = BOTH ? (int)(blockIdx.x & 1) : A.po;
+  const int block = BOTH ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, blocks = gridDim.x >> BOTH;
   const size_t in_base = (size_t)(1 - po) * nh;
   const size_t out_base = (size_t)po * nh;
-  const size_t in_off = A.both ? in_base : 0, out_off = A.both ? out_base : 0;
+  const size_t in_off = BOTH ? in_base : 0, out_off = BOTH ? out_base : 0;
   const double2 *__restrict__ xin = A.xin + in_off;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double dot = 0.0;
@@ -355,22 +364,41 @@ __global__ void __launch_bounds__(kBlock) dslash64_split_kernel(const DslashArgs
 }
 
 // Sites per launch up to which a half sweep spreads each site over a block's
-// warps: between the last lattice measured faster that way and the first
-// measured slower (Schur us, whole-site / split; fat+Naik: 24^4 145.6 / 137.9,
-// 24^3 x 32 165.5 / 185.1; naive: 16^3 x 32 39.4 / 35.6, 20^4 41.5 / 42.3).
-template <int NL>
-constexpr int kSplitMax = NL == 8 ? 196608 : 65536;
+// warps; above, a thread has a whole site, with 255 registers while there is no
+// more than one block for each SM and 128 beyond.  Between the last lattice
+// measured faster and the first slower.  Schur us, split / 255 / 128 registers:
+//   fat+Naik 12^4 12.4 / 16.1 / 21.0, 14^4 18.9 / 19.9 / 24.2, 12^3 x 32 27.7 /
+//   23.8 / 27.0, 16^4 30.8 / 26.5 / 29.1, 16^3 x 24 43.0 / 42.9 / 36.6
+//   naive 14^4 10.4 / 11.3 / 12.9, 12^3 x 32 12.5 / 12.9 / 14.6, 16^4 15.5 / 14.5 /
+//   16.2, 16^3 x 24 21.9 / 25.1 / 20.9, 24^4 61.4 / 65.8 / 61.6
+//   D, fat+Naik 8^3 x 16 5.8 / 7.2 / 9.2, 12^4 9.5 / 8.4 / 10.4, 16^4 25.8 / 18.2 / 14.7
+template <int NL, int BOTH>
+constexpr int kSplitMax = BOTH ? 16384 : NL == 8 ? 23000 : 30000;
 
-template <int NL, int HOP, int INIT, int RED>
+template <int NL, int HOP, int INIT, int RED, int BOTH = 0>
 static void launch64(const DslashArgs64 &A) {
-  const int par = A.both ? 2 : 1;  // parities in the launch
-  if (par * A.nsites <= kSplitMax<NL>) {
+  constexpr int par = BOTH + 1;  // parities in the launch
+  if (par * A.nsites <= kSplitMax<NL, BOTH>) {
     const int grid = std::min((A.nsites + kSplitSites - 1) / kSplitSites, num_sms() * 3 / par);
-    launch_pdl(dslash64_split_kernel<NL, HOP, INIT, RED>, par * grid, kBlock, A);
+    launch_pdl(dslash64_split_kernel<NL, HOP, INIT, RED, 0, BOTH>, par * grid, kBlock, A);
   } else {
-    launch_pdl(dslash64_kernel<NL, HOP, INIT, RED>, par * grid_for(A.nsites, kBlock, 6 / par), kBlock, A);
+    const int grid = par * grid_for(A.nsites, kBlock, 6 / par);
+    if (grid <= num_sms())
+      launch_pdl(dslash64_kernel<NL, HOP, INIT, RED, BOTH, 1>, grid, kBlock, A);
+    else
+      launch_pdl(dslash64_kernel<NL, HOP, INIT, RED, BOTH, 2>, grid, kBlock, A);
   }
   note_launch();
+}
+
+template <int NL>
+static void launch_both(const DslashArgs64 &A, int init) {
+  if (init == 0)
+    launch64<NL, 1, 0, kRedNone, 1>(A);
+  else if (init == 1)
+    launch64<NL, 1, 1, kRedNone, 1>(A);
+  else
+    launch64<NL, 1, 2, kRedNone, 1>(A);
 }
 
 template <int NL>
@@ -420,7 +448,6 @@ int dslash64(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, C
   A.k0 = A.k2 = 0;
   A.n1 = A.nsites = g.nh;
   A.rowlen = A.pitch = 0;
-  A.both = 0;
   int rc = (gl->nl == 8) ? dispatch64<8>(A, hop, init, red) : dispatch64<4>(A, hop, init, red);
   if (rc) return rc;
   QS_LAUNCH_CHECK();
@@ -432,9 +459,9 @@ int dslash64(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD xs, C
 // that one reads as the forward link of its own site the other reads as the
 // backward link of a site nearby: side by side, the second read finds it in
 // L2, where one launch after the other had the links from HBM twice.  D, us,
-// two launches / one: 12 x 10 x 14 x 18 fat+Naik 18.6 / 17.6, 24^4 147 / 92, 32^4
-// 411 / 386 (three time slices of links, the reach of the long hops, are most
-// of L2 there); naive 24^4 80 / 51.
+// two launches / one: 12 x 10 x 14 x 18 fat+Naik 18.2 / 9.3, 24^4 120 / 73, 32^4
+// 371 / 289 (three time slices of links, the reach of the long hops, are most
+// of L2 there); naive 24^4 61 / 37, 32^4 199 / 141.
 int dslash64_both(const qexstag_links_s *gl, double2 *out, const double2 *x, const double2 *rin, double a, double b,
                   double c, int init) {
   const Geom &g = gl->l->g;
@@ -449,9 +476,10 @@ int dslash64_both(const qexstag_links_s *gl, double2 *out, const double2 *x, con
   A.b = b;
   A.c = c;
   A.n1 = A.nsites = g.nh;
-  A.both = 1;
-  const int rc = gl->nl == 8 ? dispatch64<8>(A, +1, init, kRedNone) : dispatch64<4>(A, +1, init, kRedNone);
-  if (rc) return rc;
+  if (gl->nl == 8)
+    launch_both<8>(A, init);
+  else
+    launch_both<4>(A, init);
   QS_LAUNCH_CHECK();
   return QEXSTAG_OK;
 }
@@ -526,8 +554,15 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
   return QEXSTAG_OK;
 }
 
+// Whether an FP64 CG takes the fused iteration, whose sweeps are spread over
+// warps: on small lattices, and where the whole-site form would have a second
+// round of blocks (two on an SM) that is nearly empty.  Iteration us, fused /
+// not: fat+Naik 12^4 18 / 24.5, 12^3 x 32 32 / 36, 16^4 40.0 / 38.8, 16^3 x 32
+// 63 / 59, 20^4 (313 blocks for 296 places) 76 / 86, 24^4 151 / 147; naive 12^3 x 32
+// 21.5 / 27.3, 16^4 26.6 / 25.9, 16^3 x 32 41.5 / 38.5, 20^4 48 / 52, 24^4 87 / 85.
 bool cg_fused_fits(const qexstag_links_s *gl) {
-  return gl->l->g.nh <= (gl->nl == 8 ? kSplitMax<8> : kSplitMax<4>);
+  const int nh = gl->l->g.nh, blocks = (nh + kBlock - 1) / kBlock, places = 2 * num_sms();
+  return nh <= 30000 || (blocks > places && blocks <= places + places / 3);
 }
 
 // the two half sweeps of a fused CG iteration; *npap: the <p, Ap> partials

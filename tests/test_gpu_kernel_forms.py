@@ -17,9 +17,11 @@ def rel(a, b):
     return np.abs(a - b).max() / np.abs(b).max()
 
 
-# half sweeps: 4^4 (128 sites a parity), 720 = 22 1/2 sets of 32 sites, 65536
-# (the last naive lattice spread over warps) and 69632 (the first that is not)
+# half sweeps: 4^4 (128 sites a parity), 720 = 22 1/2 sets of 32 sites, 19208 (fat
+# +Naik: still spread over warps) and 23520 (no longer; 91 7/8 sets of 256), 40960
+# (more of them than SMs), 65536 and 69632
 @pytest.mark.parametrize("dims,naik", [((4, 4, 4, 4), 0), ((4, 6, 6, 10), 0), ((4, 6, 6, 10), 1),
+                                       ((14, 14, 14, 14), 1), ((12, 14, 14, 20), 1), ((16, 16, 16, 20), 1),
                                        ((16, 16, 16, 32), 0), ((16, 16, 16, 34), 0)])
 def test_half_sweep_forms(cuda, dims, naik):
     g = F.fat_naik_links(dims, 3) if naik else F.naive_links(dims, 0.3, 3)
@@ -150,10 +152,10 @@ def test_batch_partitions(cuda, shapes):
         assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
 
 
-# both parities in one launch, spread over warps (720 even sites) and not (69632
-# naive, 165888 fat+Naik): the same bits as one parity after the other
-@pytest.mark.parametrize("dims,naik", [((4, 6, 6, 10), 0), ((4, 6, 6, 10), 1), ((16, 16, 16, 34), 0),
-                                       ((24, 24, 24, 24), 1)])
+# both parities in one launch, spread over warps (up to 8192 even sites) and not:
+# the same bits as one parity after the other
+@pytest.mark.parametrize("dims,naik", [((4, 6, 6, 10), 0), ((4, 6, 6, 10), 1), ((8, 8, 8, 32), 1), ((8, 8, 8, 34), 1),
+                                       ((16, 16, 16, 34), 0), ((24, 24, 24, 24), 1)])
 def test_both_parities_in_one_launch(cuda, dims, naik):
     torch, V = cuda, F.volume(dims)
     gen = torch.Generator(device="cuda").manual_seed(3)
@@ -199,3 +201,19 @@ def test_several_vectors_forms(cuda, dims, n, naik):
             one = r0.clone()
             s.stagD2(par, one, x, 0.0, 0.3)
             assert float((r - one).abs().max() / one.abs().max()) < 1e-13
+
+
+# FP64 solves with the fused iteration (19208 even sites; 81648, 319 sets of 256)
+# and without it (32768 and 40960)
+@pytest.mark.parametrize("dims", [(14, 14, 14, 14), (16, 16, 16, 16), (16, 16, 16, 20), (18, 18, 18, 28)])
+@pytest.mark.parametrize("naik", [0, 1])
+def test_solve_forms(cuda, dims, naik):
+    g = F.fat_naik_links(dims, 3) if naik else F.naive_links(dims, 0.3, 3)
+    o, s = O.Oracle(dims, g), S.Staggered(S.Layout(dims), S.to_device_links(g))
+    b = F.even_source(dims, 4)
+    x, sp = S.to_device_vector(np.zeros_like(b)), S.SolverParams(r2req=1e-20)
+    s.solveEE(x, S.to_device_vector(b), 0.5, sp)
+    assert sp.status == S.L.OK and sp.r2 <= 1e-20
+    x, ax = S.to_host_vector(x), o.vec()
+    o.stagD2ee(ax, x, 0.25)
+    assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
