@@ -20,9 +20,9 @@
 // the same fixed order, so all take the same decisions without a further
 // step, and results are bitwise reproducible.  Finished problems drop out; the
 // kernel returns when none is active.  16 lattices of 2048 to 8192 even sites:
-// 8.0 ms, where a thread per site, a ticket per problem with its last block
+// 7.4 ms, where a thread per site, a ticket per problem with its last block
 // finishing the sums, and a barrier of two hops took 10.9 ms; the links through
-// L2, 150 MB an iteration while all are active, are 12 of its 34 us.
+// L2, 150 MB an iteration while all are active, are 12 of its 31 us.
 //
 // Every wait is bounded: a barrier that has not completed within the time
 // limit sets an error flag and all blocks return; the host reports
@@ -311,8 +311,12 @@ __device__ __forceinline__ void pointwise(BShared<NL> &S, F f) {
   if (lane == 0 && T.np > 0) S.red[w][i - T.i0] = acc;
 }
 
+// Two blocks on an SM: with 108 registers a warp has its link's loads in flight
+// together, where the 64 that the compiler takes without the bound (three blocks)
+// make it wait in between (16 lattices, naive, 8 x 8 x 8 x 16 and its like: 7.99 ->
+// 7.35 ms).
 template <int NL>
-__global__ void __launch_bounds__(kBatchBlock) batched_cg_kernel(const BArgs A) {
+__global__ void __launch_bounds__(kBatchBlock, 2) batched_cg_kernel(const BArgs A) {
   extern __shared__ __align__(16) unsigned char shared_bytes[];
   BShared<NL> &S = *reinterpret_cast<BShared<NL> *>(shared_bytes);
   const int nprob = A.set->nprob, maxits = A.set->maxits;
