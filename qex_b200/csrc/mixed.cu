@@ -318,9 +318,9 @@ __device__ __forceinline__ bool mx_test(MxState *st, double r2, int itn) {
 // are kept apart so that the FP16 list scales multiply them once per site.
 // ---------------------------------------------------------------------------
 
-// dslash_lo_kernel serves the FP32 links (it runs at the copy bandwidth with
-// its natural registers); 16-bit links go to dslash_x2_kernel below.  The
-// 16-bit kernel is instruction-heavy for the bytes it moves and gains from
+// dslash_lo_kernel serves the FP32 links (it runs at the copy bandwidth);
+// 16-bit links go to dslash_x2_kernel below.  On large lattices the 16-bit
+// kernel is instruction-heavy for the bytes it moves and gains from
 // occupancy: 4 resident blocks of 64 registers (with scalar arithmetic this
 // gave 4450 GB/s on 32^4 against 4090 GB/s at 72-80 registers; splitting a
 // site's forward and backward hops over two threads gave 3640-3720 GB/s).
@@ -359,8 +359,8 @@ struct DslashArgsLo {
   Progress progress;  // posted by this launch (a solve's first half sweep)
 };
 
-template <int PREC, int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12>
-__global__ void __launch_bounds__(kBlock, PREC == kF16 ? 4 : 1) dslash_lo_kernel(const DslashArgsLo A) {
+template <int PREC, int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12, int RESIDENT>
+__global__ void __launch_bounds__(kBlock, RESIDENT) dslash_lo_kernel(const DslashArgsLo A) {
   pdl_wait();
   post_progress(A.progress);
   if (A.halt != nullptr && mx_halt(A.halt)) return;
@@ -482,8 +482,8 @@ __global__ void __launch_bounds__(kBlock, PREC == kF16 ? 4 : 1) dslash_lo_kernel
 // decoded directly as -conj(U) (its row 2 rebuilt with -k) so that its
 // terms add.  The long hops' vectors are scaled by long_scale / fat_scale,
 // so one set of accumulators carries both lists in fat units.
-template <int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12>
-__global__ void __launch_bounds__(kBlock, 4) dslash_x2_kernel(const DslashArgsLo A) {
+template <int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12, int RESIDENT>
+__global__ void __launch_bounds__(kBlock, RESIDENT) dslash_x2_kernel(const DslashArgsLo A) {
   pdl_wait();
   post_progress(A.progress);
   if (A.halt != nullptr && mx_halt(A.halt)) return;
@@ -600,57 +600,43 @@ __global__ void __launch_bounds__(kBlock, 4) dslash_x2_kernel(const DslashArgsLo
   }
 }
 
-// Grid of a sloppy half sweep.  The 16-bit kernel runs exactly two waves of
-// resident blocks (occupancy from the runtime, so that no partial wave idles
-// SMs: on 32^4 two waves gave 5208 GB/s, 1.5 waves 4437); the FP32 kernel is
-// at the copy bandwidth with 4 blocks per SM.
+// Launches a sloppy half sweep on n sites; returns the grid.  While an SM has one
+// block, the kernel is one that may take all registers, for the loads of several
+// hops at once; with two blocks an SM, half of them.  Beyond, the FP32 kernel keeps
+// that half, in two waves, and the 16-bit kernel, which is then bound by its
+// instructions, takes two waves of four blocks (no partial wave idles SMs: on 32^4
+// two waves gave 5208 GB/s, 1.5 waves 4437).  CG iteration, us:
+//   16 bits, four blocks an SM / this rule: fat+Naik 12^3 x 32 24.5 / 20.0, 16^4 26.1 /
+//   20.8, 16^3 x 20 29.0 / 24.6, 16^3 x 32 29.5 / 25.8; naive 16^4 17.1 / 16.0
+//   FP32, one block an SM / two / three: fat+Naik 16^4 21.4 / 23.9 / 30.0, 24^4 77.0 /
+//   75.0 / 76.1, 32^4 220 / 217 / 230; naive 16^4 14.3 / 15.8 / 17.5, 24^4 49.7 / 45.4 /
+//   44.8, 32^4 129 / 123 / 125
 template <int PREC, int VP, int NL, int HOP, int INIT, int RED, int OUTP, int R12>
-static int lo_grid(int nh) {
-  static int resident = 0;  // one per kernel instantiation
-  if (resident == 0) {
-    int n = 0;
-    cudaError_t e;
+static int launch_lo_n(const DslashArgsLo &A, int n) {
+  const int sets = std::max(1, (n + kBlock - 1) / kBlock);
+  if (sets <= num_sms()) {
     if constexpr (PREC == kF16)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, R12>,
-                                                        kBlock, 0);
+      launch_pdl(dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, R12, 1>, sets, kBlock, A);
     else
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dslash_lo_kernel<PREC, VP, NL, HOP, INIT, RED, OUTP, R12>,
-                                                        kBlock, 0);
-    if (e != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = 4;
-    }
-    resident = n;
+      launch_pdl(dslash_lo_kernel<PREC, VP, NL, HOP, INIT, RED, OUTP, R12, 1>, sets, kBlock, A);
+    return sets;
   }
-  long want = (long)num_sms() * (PREC == kF16 ? 2 * resident : 4);
-  long need = (nh + kBlock - 1) / kBlock;
-  long g = want < need ? want : need;
-  if (g > kMaxRedBlocks) g = kMaxRedBlocks;
-  return (int)(g < 1 ? 1 : g);
+  const int grid = std::min({sets, num_sms() * (PREC == kF16 ? 8 : 4), kMaxRedBlocks});
+  if constexpr (PREC == kF32)
+    launch_pdl(dslash_lo_kernel<PREC, VP, NL, HOP, INIT, RED, OUTP, R12, 2>, grid, kBlock, A);
+  else if (sets <= 2 * num_sms())
+    launch_pdl(dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, R12, 2>, grid, kBlock, A);
+  else
+    launch_pdl(dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, R12, 4>, grid, kBlock, A);
+  return grid;
 }
 
-// returns the grid launched
 template <int PREC, int VP, int NL, int HOP, int INIT, int RED, int OUTP>
 static int launch_lo(const DslashArgsLo &A, int) {
-  int grid;
-  const int nsites = std::max(0, std::min(A.g.nh, A.k_hi) - A.k_lo);
-  if constexpr (PREC == kF16) {
-    if (NL == 8 && A.L.recon12) {
-      grid = lo_grid<PREC, VP, NL, HOP, INIT, RED, OUTP, 1>(nsites);
-      launch_pdl(dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, 1>, grid, kBlock, A);
-    } else {
-      grid = lo_grid<PREC, VP, NL, HOP, INIT, RED, OUTP, 0>(nsites);
-      launch_pdl(dslash_x2_kernel<VP, NL, HOP, INIT, RED, OUTP, 0>, grid, kBlock, A);
-    }
-  } else if (NL == 8 && A.L.recon12) {
-    grid = lo_grid<PREC, VP, NL, HOP, INIT, RED, OUTP, 1>(nsites);
-    launch_pdl(dslash_lo_kernel<PREC, VP, NL, HOP, INIT, RED, OUTP, 1>, grid, kBlock, A);
-  } else {
-    grid = lo_grid<PREC, VP, NL, HOP, INIT, RED, OUTP, 0>(nsites);
-    launch_pdl(dslash_lo_kernel<PREC, VP, NL, HOP, INIT, RED, OUTP, 0>, grid, kBlock, A);
-  }
+  const int n = std::max(0, std::min(A.g.nh, A.k_hi) - A.k_lo);
   note_launch();
-  return grid;
+  return NL == 8 && A.L.recon12 ? launch_lo_n<PREC, VP, NL, HOP, INIT, RED, OUTP, 1>(A, n)
+                                : launch_lo_n<PREC, VP, NL, HOP, INIT, RED, OUTP, 0>(A, n);
 }
 
 // the two half sweeps of the sloppy Schur operator:

@@ -217,3 +217,20 @@ def test_solve_forms(cuda, dims, naik):
     x, ax = S.to_host_vector(x), o.vec()
     o.stagD2ee(ax, x, 0.25)
     assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
+
+
+# reduced-precision half sweeps by blocks on an SM: 36864 even sites are 144 sets
+# of 256 (one block an SM), 40960 are 160 (two), 81648 are 318 15/16 (four)
+@pytest.mark.parametrize("dims", [(16, 16, 16, 18), (16, 16, 16, 20), (18, 18, 18, 28)])
+@pytest.mark.parametrize("sloppy", [1, 2])
+@pytest.mark.parametrize("naik", [0, 1])
+def test_reduced_precision_forms(cuda, dims, sloppy, naik):
+    g = F.fat_naik_links(dims, 3) if naik else F.naive_links(dims, 0.3, 3)
+    o, s = O.Oracle(dims, g), S.Staggered(S.Layout(dims), S.to_device_links(g))
+    b = F.even_source(dims, 4)
+    x, sp = S.to_device_vector(np.zeros_like(b)), S.SolverParams(r2req=1e-20, sloppySolve=sloppy)
+    s.solveEE(x, S.to_device_vector(b), 0.5, sp)
+    assert sp.status == S.L.OK and sp.r2 <= 1e-20
+    x, ax = S.to_host_vector(x), o.vec()
+    o.stagD2ee(ax, x, 0.25)
+    assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
