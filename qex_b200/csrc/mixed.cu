@@ -832,7 +832,9 @@ __global__ void __launch_bounds__(kBlock)
                        const void *pin, void *pout, int n, MxState *st, const double *pap, const double *apap,
                        int np, const double *r2in, int nr2, double *r2out, int par, const double *rap = nullptr) {
   pdl_wait();
-  if (mx_halt(st)) return;
+  // block 0 may be setting the flags: one answer for all threads of a block,
+  // or a sum below would lack the part of those that left
+  if (__syncthreads_or(mx_halt(st))) return;
   // the first site's operands are loaded before the sums of the partials,
   // so that their latencies overlap
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
