@@ -122,9 +122,9 @@ __device__ __forceinline__ void reduce_pap(const DslashArgs64 &A, double dot) {
 // fat+Naik 32^4 423 / 374 / 380, 24^4 146 / 121 / 121, 16^4 64 / 29 / 26.5; naive
 // 32^4 224 / 190 / 196, 24^4 79 / 62 / 66; D fat+Naik 32^4 361 / 289 / 291, naive
 // 208 / 141 / 145; an FP64 CG iteration at 32^4 fat+Naik 534 / 424 / 427, naive 286
-// / 241 / 247.  At 32^4 fat+Naik the Schur operator moves its compulsory bytes at
-// 6.8 TB/s, above the copy rate: part of the links is still in L2 from the other
-// sweep.  A block for every 256 sites instead of six per SM: 379.
+// / 241 / 247.  At 32^4 fat+Naik a half sweep then reads its compulsory bytes, and
+// no more, from HBM at 6.9 TB/s, above the copy rate.  A block for every 256 sites
+// instead of six per SM: 379.
 template <int NL, int HOP, int INIT, int RED, int BOTH, int RESIDENT>
 __global__ void __launch_bounds__(kBlock, RESIDENT) dslash64_kernel(const DslashArgs64 A) {
   pdl_wait();
