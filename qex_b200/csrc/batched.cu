@@ -35,20 +35,16 @@
 #include <mutex>
 #include <vector>
 
+#include "batch_part.cuh"
 #include "lib.cuh"
 
 namespace qs {
 
 int cg64(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, double r2req, int maxits, CgOut *out);
 
-constexpr int kMaxBatch = 128;
-
 constexpr int kBatchBlock = 256;
 constexpr int kBatchWarps = kBatchBlock / 32;
 constexpr int kSetSites = 32;
-// problems that one block's chunk meets: a problem has at least 4 sets (4^4),
-// so 128 of them spread over more than two blocks never put more in one
-constexpr int kMaxMet = 64;
 
 struct BProb {
   Geom g;
@@ -134,19 +130,6 @@ __global__ void barrier_selftest_kernel(BGlobal *gl, long long timeout, unsigned
   if (blockIdx.x == 0 && threadIdx.x == 0) *out = (a && b) ? 1 : 0;
 }
 
-// The partition: the still-active problems (ids, in order), soff[i] the first
-// set of the i-th, cut into equal contiguous chunks, one to each of the first
-// nb blocks.  Every block builds the same table.
-struct BPart {
-  int na;      // active problems
-  int ntot;    // their sets
-  int nb;      // blocks with a chunk
-  int s0, s1;  // this block's sets
-  int i0, np;  // the first problem that it meets, and how many
-  int ids[kMaxBatch];
-  int soff[kMaxBatch + 1];
-};
-
 template <int NL>
 struct BShared {
   static constexpr int kBufs = NL == 4 ? 2 : 1;
@@ -164,30 +147,10 @@ __device__ __forceinline__ int sets_of(int nh) { return (nh + kSetSites - 1) / k
 template <int NL>
 __device__ void build_part(BShared<NL> &S, int nprob) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    BPart &T = S.T;
-    int n = 0, off = 0;
-    for (int j = 0; j < nprob; j++) {
-      if (S.done[j]) continue;
-      T.ids[n] = j;
-      T.soff[n] = off;
-      off += sets_of(S.prob[j].g.nh);
-      n++;
-    }
-    T.soff[n] = off;
-    T.na = n;
-    T.ntot = off;
-    T.nb = min((int)gridDim.x, off);
-    const int b = blockIdx.x;
-    T.s0 = b < T.nb ? (int)((long long)b * off / T.nb) : off;
-    T.s1 = b < T.nb ? (int)((long long)(b + 1) * off / T.nb) : off;
-    T.i0 = T.np = 0;
-    if (T.s0 < T.s1) {
-      while (T.soff[T.i0 + 1] <= T.s0) T.i0++;
-      T.np = 1;
-      while (T.soff[T.i0 + T.np] < T.s1) T.np++;
-    }
-  }
+  if (threadIdx.x == 0)
+    fill_part(
+        S.T, nprob, [&](int j) { return S.done[j]; }, [&](int j) { return sets_of(S.prob[j].g.nh); }, gridDim.x,
+        blockIdx.x);
   __syncthreads();
 }
 
@@ -204,8 +167,7 @@ __device__ __forceinline__ void leave_partials(BShared<NL> &S, double *part, int
 }
 // the sum of active problem i's partials, by one warp, in every lane
 __device__ __forceinline__ double sum_partials(const BPart &T, const double *part, int i) {
-  const int b0 = (int)(((long long)(T.soff[i] + 1) * T.nb - 1) / T.ntot);
-  const int b1 = (int)(((long long)T.soff[i + 1] * T.nb - 1) / T.ntot);
+  const int b0 = block_of(T, T.soff[i]), b1 = block_of(T, T.soff[i + 1] - 1);
   double v = 0.0;
   for (int b = b0 + (threadIdx.x & 31); b <= b1; b += 32) v += __ldcg(part + b + i);
 #pragma unroll

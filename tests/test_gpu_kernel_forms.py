@@ -234,3 +234,27 @@ def test_reduced_precision_forms(cuda, dims, sloppy, naik):
     x, ax = S.to_host_vector(x), o.vec()
     o.stagD2ee(ax, x, 0.25)
     assert np.linalg.norm((ax - b)[: F.volume(dims) // 2]) <= 1.01e-10 * np.linalg.norm(b)
+
+
+# a batch whose large lattices make a block's chunk take in all 68 small ones:
+# each problem ends as it does by itself, without a correction
+@pytest.mark.parametrize("naik", [0, 1])
+def test_batch_of_large_and_small_lattices(cuda, naik):
+    links = F.fat_naik_links if naik else (lambda dims, seed: F.naive_links(dims, 0.3, seed))
+    kinds = []
+    for dims, n in (((16, 16, 16, 16), 60), ((4, 4, 4, 4), 68)):
+        lay, g = S.Layout(dims), S.to_device_links(links(dims, 3))
+        b = S.to_device_vector(F.even_source(dims, 4))
+        kinds += [(lay, g, b)] * n
+    ops = [S.Staggered(lay, g) for lay, g, _ in kinds]
+    xs, sp = [cuda.zeros_like(b) for _, _, b in kinds], S.SolverParams(r2req=1e-20)
+    out = S.solve_batched(ops, xs, [b for _, _, b in kinds], [0.3] * len(ops), sp)
+    assert sp.status == S.L.OK and (out["r2"] <= 1e-20).all() and sp.outer_iterations == 0
+    for j in (0, len(ops) - 1):
+        one = S.SolverParams(r2req=1e-20)
+        ops[j].solveEE(cuda.zeros_like(xs[j]), kinds[j][2], 0.3, one)
+        same = range(60) if j == 0 else range(60, 128)
+        assert all(abs(out["iterations"][i] - one.iterations) <= 1 for i in same)
+        # two solutions to |r| <= 1e-10 |b|, and 4 m^2 = 0.36 below every eigenvalue
+        far = 2e-10 * float(kinds[j][2].norm()) / 0.36
+        assert all(float((xs[i] - xs[j]).norm()) <= far for i in same)
