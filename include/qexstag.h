@@ -33,8 +33,9 @@
  *    already carry the staggered phases and boundary signs (QEX's
  *    setBC + stagPhase, src/physics/stagD.nim:106-114, 560-571).
  *  - Calls on one handle are not reentrant; separate handles and separate
- *    devices may be used from separate threads.  Work is issued on the
- *    stream set by qexstag_set_stream (default: the legacy default stream).
+ *    devices may be used from separate threads, on one stream or on several.
+ *    Work is issued on the stream that the calling thread has set with
+ *    qexstag_set_stream (default: the legacy default stream).
  */
 #ifndef QEXSTAG_H
 #define QEXSTAG_H

@@ -285,8 +285,9 @@ int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t e, const char *what);
 cudaStream_t stream();
 int num_sms();
-// Scratch for reductions: partial sums and tickets, reused by every call on
-// the library's stream (calls on one stream are ordered).
+// Scratch for reductions, the calling thread's own on the current device:
+// partial sums and tickets, reused by its calls one after the other (a call that
+// reduces waits for its result).
 double *red_partials();   // kMaxRedBlocks * 8 doubles
 unsigned *red_tickets();  // kNumTickets unsigned, all zero between kernels
 constexpr int kMaxRedBlocks = 4096;

@@ -258,3 +258,50 @@ def test_batch_of_large_and_small_lattices(cuda, naik):
         # two solutions to |r| <= 1e-10 |b|, and 4 m^2 = 0.36 below every eigenvalue
         far = 2e-10 * float(kinds[j][2].norm()) / 0.36
         assert all(float((xs[i] - xs[j]).norm()) <= far for i in same)
+
+
+# separate handles from separate threads, on the default stream and on streams
+# of their own: every solve ends as it does alone, bit for bit
+@pytest.mark.parametrize("streams", [0, 1])
+def test_solves_from_several_threads(cuda, streams):
+    import threading
+    dims = (4, 6, 6, 10)
+    b = S.to_device_vector(F.even_source(dims, 4))
+    lay, g = S.Layout(dims), S.to_device_links(F.fat_naik_links(dims, 3))
+
+    def work(s, scale):
+        out = []
+        s.update_links(g * scale)
+        for sloppy in (S.L.SLOPPY_NONE, S.L.SLOPPY_SINGLE, S.L.SLOPPY_HALF):
+            x, sp = cuda.zeros_like(b), S.SolverParams(r2req=1e-20, sloppySolve=sloppy)
+            s.solveEE(x, b, 0.1, sp)
+            out += [x, sp.iterations]
+        ys = [[cuda.zeros_like(b) for _ in range(2)] for _ in range(3)]
+        sp = S.SolverParams(r2req=1e-20, sloppySolve=S.L.SLOPPY_SINGLE)
+        out.append(s.cgm_ee(0.1, [0.0, 0.5], [b, 2.0 * b, b], ys, sp).tolist())
+        return out + [y for row in ys for y in row] + [sp.iterations]
+
+    scales = [1.0, 0.9, 1.1, 0.8]
+    ops = [S.Staggered(lay, g) for _ in scales]
+    alone = [work(s, c) for s, c in zip(ops, scales)]
+    got, start = [[] for _ in scales], threading.Barrier(len(scales))
+
+    def thread(i):
+        with cuda.cuda.stream(cuda.cuda.Stream() if streams else cuda.cuda.default_stream()):
+            S.L.load().qexstag_set_stream(cuda.cuda.current_stream().cuda_stream)
+            start.wait()
+            for _ in range(5):
+                got[i].append(work(ops[i], scales[i]))
+            cuda.cuda.current_stream().synchronize()
+
+    cuda.cuda.synchronize()
+    threads = [threading.Thread(target=thread, args=(i,)) for i in range(len(scales))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for one, runs in zip(alone, got):
+        assert len(runs) == 5
+        for run in runs:
+            for u, v in zip(one, run):
+                assert cuda.equal(u, v) if cuda.is_tensor(u) else u == v
