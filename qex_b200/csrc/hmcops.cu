@@ -409,10 +409,13 @@ static int rect_force_dev(qexstag_layout_s *l, const double2 *u, double2 *f, dou
   const Geom &g = l->g;
   const int T = g.L[3], sh = g.nh / T;  // half sites of a time slice
   const size_t slice = (size_t)24 * 9 * sizeof(double2) * 2 * sh;
-  int n = T;  // slices of force per slab
-  if (slice * T > kGaugeScratch) n = std::max(1, std::min(T, (int)(kGaugeScratch / slice) - 3));
-  const int held = std::min(T, n + 3);  // slices of scratch
-  if (n == 1 && held == 4 && T > 4 && slice * held > kGaugeScratch) return QEXSTAG_ERR_ALLOC;
+  // slices of force per slab, and of scratch
+  int n = T, held = T;
+  if (slice * T > kGaugeScratch) {
+    held = (int)(kGaugeScratch / slice);  // < T
+    n = held - 3;
+    if (n < 1) return QEXSTAG_ERR_ALLOC;
+  }
   void *p = l->scratch.take(slice * held);
   if (!p) return QEXSTAG_ERR_ALLOC;
   GaugeArgs A;
