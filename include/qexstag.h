@@ -451,7 +451,10 @@ int qexstag_gauge_action(qexstag_layout *l, const qexstag_gauge_coefs *c, const 
 /* gaugeForce (gaugeAction.nim:576-779): f_mu(x) = projectTAH(U_mu(x) C_mu(x)),
    C the plaq/3- and rect/3-weighted sums of the paths that close each
    plaquette and rectangle through U_mu(x); along U -> exp(t T) U the action
-   changes at rate Re Tr[T^dag f]. */
+   changes at rate Re Tr[T^dag f].  With rectangles, up to 4 GiB of device
+   scratch (3456 B per site) stays with the layout for the next force; it is
+   freed with the layout, or when another allocation of the library would fail
+   without it.  Where it cannot be had the force takes a slower form. */
 int qexstag_gauge_force(qexstag_layout *l, const qexstag_gauge_coefs *c, const double *u, double *f, int mem);
 /* axexpmuly(u, eps, p, u) (gaugeUtils.nim:452-459): u <- expAH(eps p) u with
    QEX's expAH (scaling, degree-12 Taylor, squaring; matexp.nim:316-346). */

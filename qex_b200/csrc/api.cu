@@ -25,26 +25,68 @@ int stagD_par(qexstag_links_s *g, int par, double2 *r, const double2 *x, double 
               double a);
 int rephase_links(qexstag_links_s *g, bool literal);
 
+namespace {
+// every pool of the process (never destroyed: a layout may outlive the
+// process's static objects)
+std::mutex &g_pools_mutex = *new std::mutex;
+std::vector<ScratchPool *> &g_pools = *new std::vector<ScratchPool *>;
+
+int this_device() {
+  int d = 0;
+  cudaGetDevice(&d);
+  return d;
+}
+}  // namespace
+
+ScratchPool::ScratchPool() {
+  std::lock_guard<std::mutex> lock(g_pools_mutex);
+  g_pools.push_back(this);
+}
+
+ScratchPool::~ScratchPool() {
+  {
+    std::lock_guard<std::mutex> lock(g_pools_mutex);
+    g_pools.erase(std::find(g_pools.begin(), g_pools.end(), this));
+  }
+  for (Buf &b : bufs_) cudaFree(b.p);
+}
+
+void ScratchPool::free_idle() {
+  const int d = this_device();
+  std::lock_guard<std::mutex> all(g_pools_mutex);
+  for (ScratchPool *q : g_pools) {
+    std::lock_guard<std::mutex> lock(q->m_);
+    for (size_t i = q->bufs_.size(); i-- > 0;)
+      if (!q->bufs_[i].used && q->bufs_[i].device == d) {
+        cudaFree(q->bufs_[i].p);
+        q->bufs_.erase(q->bufs_.begin() + i);
+      }
+  }
+}
+
 void *ScratchPool::take(size_t bytes) {
-  std::lock_guard<std::mutex> lock(m_);
-  for (Buf &b : bufs_)
-    if (!b.used && b.bytes >= bytes) {
-      b.used = true;
-      return b.p;
-    }
-  // a free buffer that is too small makes way
-  for (size_t i = 0; i < bufs_.size(); i++)
-    if (!bufs_[i].used) {
-      cudaFree(bufs_[i].p);
-      bufs_.erase(bufs_.begin() + i);
-      break;
-    }
+  {
+    std::lock_guard<std::mutex> lock(m_);
+    for (Buf &b : bufs_)
+      if (!b.used && b.bytes >= bytes) {
+        b.used = true;
+        return b.p;
+      }
+    // a free buffer that is too small makes way
+    for (size_t i = 0; i < bufs_.size(); i++)
+      if (!bufs_[i].used) {
+        cudaFree(bufs_[i].p);
+        bufs_.erase(bufs_.begin() + i);
+        break;
+      }
+  }
   void *p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+  if (device_malloc(&p, bytes) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  bufs_.push_back(Buf{p, bytes, true});
+  std::lock_guard<std::mutex> lock(m_);
+  bufs_.push_back(Buf{p, bytes, this_device(), true});
   return p;
 }
 
@@ -52,10 +94,6 @@ void ScratchPool::give(void *p) {
   std::lock_guard<std::mutex> lock(m_);
   for (Buf &b : bufs_)
     if (b.p == p) b.used = false;
-}
-
-ScratchPool::~ScratchPool() {
-  for (Buf &b : bufs_) cudaFree(b.p);
 }
 
 int Workspace::get(int slot, size_t bytes, void **out) {
@@ -70,7 +108,7 @@ int Workspace::get(int slot, size_t bytes, void **out) {
     bufs.erase(it);
   }
   void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
+  cudaError_t e = device_malloc(&p, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, std::string("device allocation of ") + std::to_string(bytes) +
@@ -320,7 +358,7 @@ int qexstag_layout_shift_table(const qexstag_layout *l, int mu, int len, int sub
   const Geom &g = l->g;
   int n = subset == 2 ? g.V : g.nh;
   int32_t *d = nullptr;
-  QS_CUDA(cudaMalloc(&d, sizeof(int32_t) * n));
+  QS_CUDA(device_malloc(&d, sizeof(int32_t) * n));
   shift_table_kernel<<<grid_for(n), kBlock, 0, stream()>>>(g, mu, len, subset, n, d);
   note_launch();
   cudaError_t e = cudaGetLastError();
@@ -426,7 +464,7 @@ int qexstag_links_create(qexstag_layout *l, int nlinks, const double *links, int
   g->long_coeff = long_coeff;
   const Geom &geo = l->g;
   const size_t per = sizeof(double2) * 9 * (size_t)geo.V;
-  cudaError_t e = cudaMalloc(&g->u64, per * nlinks);
+  cudaError_t e = device_malloc(&g->u64, per * nlinks);
   if (e != cudaSuccess) {
     cudaGetLastError();
     delete g;
@@ -491,7 +529,7 @@ int qexstag_links_create_milc(qexstag_layout *l, const double *fat, const double
   g->nl = nl;
   g->long_coeff = long_coeff;
   const size_t per = sizeof(double2) * 9 * (size_t)l->g.V;
-  cudaError_t e = cudaMalloc(&g->u64, per * nl);
+  cudaError_t e = device_malloc(&g->u64, per * nl);
   if (e != cudaSuccess) {
     cudaGetLastError();
     delete g;

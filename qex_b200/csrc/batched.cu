@@ -606,7 +606,7 @@ int solve_batched(int nprob, qexstag_links_s *const *gs, const double *mass, dou
     }
     if (bc->exec) cudaGraphExecDestroy(bc->exec);
     bc->exec = nullptr;
-    cudaError_t e = cudaMalloc(&bc->arena, bytes);
+    cudaError_t e = device_malloc(&bc->arena, bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       bc->arena = nullptr;
@@ -725,7 +725,7 @@ int qexstag_barrier_selftest(int missing, double timeout_ms) {
   const long long cycles = (long long)(timeout_ms * (double)khz);  // kHz x ms = cycles
   BGlobal *gl = nullptr;
   int *out = nullptr;
-  if (cudaMalloc(&gl, sizeof(BGlobal)) != cudaSuccess || cudaMalloc(&out, sizeof(int)) != cudaSuccess) {
+  if (device_malloc(&gl, sizeof(BGlobal)) != cudaSuccess || device_malloc(&out, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     if (gl) cudaFree(gl);
     return fail(QEXSTAG_ERR_ALLOC, "barrier_selftest: allocation failed");

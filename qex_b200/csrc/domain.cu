@@ -907,7 +907,7 @@ static int domain_create(const int global_dims[4], int Rz, int Rt, int rank, int
   qexstag_layout_destroy(ll);
   void *z = nullptr;
   const size_t lb = sizeof(double2) * 9 * (size_t)le->g.V * nlinks;
-  if (cudaMalloc(&z, lb) != cudaSuccess || cudaMalloc((void **)&d->dsum, kDevScalarBytes) != cudaSuccess ||
+  if (device_malloc(&z, lb) != cudaSuccess || device_malloc(&d->dsum, kDevScalarBytes) != cudaSuccess ||
       cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming) != cudaSuccess) {

@@ -327,7 +327,7 @@ static int crc_tables_dev(uint32_t **out) {
     CrcTables h;
     make_crc_tables(h);
     void *p;
-    if (cudaMalloc(&p, sizeof h) != cudaSuccess) {
+    if (device_malloc(&p, sizeof h) != cudaSuccess) {
       cudaGetLastError();
       return fail(QEXSTAG_ERR_ALLOC, "gauge I/O: table allocation failed");
     }
@@ -345,7 +345,7 @@ static int run_io_kernel(const Geom &g, uint8_t *payload, double2 *links, int pr
   int rc;
   if ((rc = crc_tables_dev(&tables))) return rc;
   DevBuf sums;
-  if (cudaMalloc(&sums.p, 2 * sizeof(unsigned)) != cudaSuccess) {
+  if (device_malloc(&sums.p, 2 * sizeof(unsigned)) != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, "gauge I/O: allocation failed");
   }
@@ -430,7 +430,7 @@ static int links_in(const Geom &g, const double *links, int mem, DevBuf &own, do
     *dev = (double2 *)links;
     return QEXSTAG_OK;
   }
-  if (cudaMalloc(&own.p, 5 * per) != cudaSuccess) {
+  if (device_malloc(&own.p, 5 * per) != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, "gauge I/O: allocation failed");
   }
@@ -650,7 +650,7 @@ int qexstag_gauge_read(qexstag_layout *l, const char *path, double *links, int m
   const uint64_t want = (uint64_t)g.V * 72 * fi.prec;
   if (fi.data_len != want) return fail(QEXSTAG_ERR_IO, "gauge_read: binary record has the wrong length");
   DevBuf payload, own;
-  if (cudaMalloc(&payload.p, want) != cudaSuccess) {
+  if (device_malloc(&payload.p, want) != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, "gauge_read: allocation failed");
   }
@@ -685,7 +685,7 @@ int qexstag_gauge_write(qexstag_layout *l, const char *path, const double *links
   const Geom &g = l->g;
   const uint64_t nbytes = (uint64_t)g.V * 72 * precision;
   DevBuf payload, own;
-  if (cudaMalloc(&payload.p, nbytes) != cudaSuccess) {
+  if (device_malloc(&payload.p, nbytes) != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, "gauge_write: allocation failed");
   }

@@ -658,7 +658,7 @@ static int field_in(const Geom &g, const double *p, int mem, bool upload, Field4
     return QEXSTAG_OK;
   }
   const size_t per = sizeof(double2) * 9 * (size_t)g.V;
-  if (cudaMalloc(&f.own, 5 * per) != cudaSuccess) {
+  if (device_malloc(&f.own, 5 * per) != cudaSuccess) {
     cudaGetLastError();
     return fail(QEXSTAG_ERR_ALLOC, "device allocation failed");
   }

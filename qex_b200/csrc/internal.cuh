@@ -348,17 +348,34 @@ class ScratchPool {
  public:
   void *take(size_t bytes);  // null when it cannot be had
   void give(void *p);
+  ScratchPool();
   ~ScratchPool();
+  // frees the buffers that no call holds, of all pools on the current device
+  static void free_idle();
 
  private:
   struct Buf {
     void *p;
     size_t bytes;
+    int device;
     bool used;
   };
   std::mutex m_;
   std::vector<Buf> bufs_;
 };
+
+// cudaMalloc; where memory is short, once more without the pools' idle buffers,
+// so that no allocation fails for what is only kept for a later call
+template <class T>
+inline cudaError_t device_malloc(T **p, size_t bytes) {
+  cudaError_t e = cudaMalloc((void **)p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    ScratchPool::free_idle();
+    e = cudaMalloc((void **)p, bytes);
+  }
+  return e;
+}
 }  // namespace qs
 
 // handles

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kBlock) low_copy_kernel(const double2 *__restr
 template <class T>
 static int dalloc(T **p, size_t n) {
   if (*p) return QEXSTAG_OK;
-  cudaError_t e = cudaMalloc((void **)p, sizeof(T) * n);
+  cudaError_t e = device_malloc(p, sizeof(T) * n);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;

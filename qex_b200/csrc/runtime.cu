@@ -67,7 +67,7 @@ int current_device() {
 int add_scratch(DeviceRuntime &r) {
   Scratch c;
   cudaStream_t s = nullptr;
-  cudaError_t e = cudaMalloc(&c.partials, sizeof(double) * kScratchDoubles);
+  cudaError_t e = device_malloc(&c.partials, sizeof(double) * kScratchDoubles);
   if (e == cudaSuccess) e = cudaHostAlloc(&c.host_results, sizeof(double) * kNumResults, cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemsetAsync(c.partials, 0, sizeof(double) * kScratchDoubles, s);

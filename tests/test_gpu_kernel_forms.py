@@ -327,3 +327,23 @@ def test_rectangle_force_scratch_of_few_slices(cuda):
     ft = torch.empty_like(u)
     MD.GaugeAction(S.Layout(turned), 5.6, -0.331).force(u, ft)
     assert float((f - ft).abs().max() / ft.abs().max()) < 1e-12
+
+
+# with the device nearly full: links are allocated in the place of the scratch
+# (1.15 GB at 24^4) that a layout keeps from its last force, and a force that
+# finds no room for its scratch goes path by path
+def test_force_scratch_makes_way(cuda):
+    torch, dims = cuda, (24, 24, 24, 24)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    u = torch.view_as_complex(torch.randn((8, 3, 3, F.volume(dims), 2), dtype=torch.float64, device="cuda",
+                                          generator=gen))
+    lay, f1, f2 = S.Layout(dims), torch.empty_like(u[:4]), torch.empty_like(u[:4])
+    MD.GaugeAction(lay, 5.6, -0.331).force(u[:4], f1)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8, device="cuda")
+    assert torch.cuda.mem_get_info()[0] < (320 << 20)
+    ops = S.Staggered(lay, u)  # 382 MB of links and their copies in less precision
+    MD.GaugeAction(S.Layout(dims), 5.6, -0.331).force(u[:4], f2)
+    del fill, ops
+    assert float((f1 - f2).abs().max() / f1.abs().max()) < 1e-12
