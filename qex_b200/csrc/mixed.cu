@@ -1551,6 +1551,7 @@ extern "C" int qexstag_bench_schur(qexstag_links *g, int prec, int nrep, double 
                                    double *seconds_per_call) {
   if (!g || !g->u64 || !seconds_per_call || nrep < 1 || prec < 0 || prec > 2)
     return qs::fail(QEXSTAG_ERR_ARG, "bench_schur: bad argument");
+  if (prec > 0 && !g->low.ready) return qs::fail(QEXSTAG_ERR_STATE, "bench_schur: reduced-precision links missing");
   int rc = qs::runtime_ready();
   if (rc) return rc;
   return qs::bench_schur(g, prec, nrep, m2, seconds_per_call);

@@ -878,6 +878,8 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
   const double m2 = m * m + 0.25 * sigma[k0];
   const int maxits = p->maxits > 0 ? p->maxits : 50000;
   const bool sloppy = p->sloppy != QEXSTAG_SLOPPY_NONE;
+  // (a failed update of the links leaves older copies, or none)
+  if (sloppy && !g->low.ready) return fail(QEXSTAG_ERR_STATE, "reduced-precision links missing");
   int rc;
   // zero the odd halves of the outputs
   for (int i = 0; i < nrhs * nshift; i++)

@@ -347,3 +347,29 @@ def test_force_scratch_makes_way(cuda):
     MD.GaugeAction(S.Layout(dims), 5.6, -0.331).force(u[:4], f2)
     del fill, ops
     assert float((f1 - f2).abs().max() / f1.abs().max()) < 1e-12
+
+
+# links that cannot be copied to less precision (all zero): the update says so,
+# and nothing goes on with the copies of the links before them
+def test_no_reduced_precision_after_a_failed_update(cuda):
+    dims = (4, 6, 6, 10)
+    g = S.to_device_links(F.fat_naik_links(dims, 3))
+    s, b = S.Staggered(S.Layout(dims), g), S.to_device_vector(F.even_source(dims, 4))
+
+    def shifted():
+        ys = [[cuda.zeros_like(b)] for _ in range(2)]
+        sp = S.SolverParams(r2req=1e-20, sloppySolve=S.L.SLOPPY_SINGLE)
+        s.cgm_ee(0.3, [0.0], [b, 2.0 * b], ys, sp)
+        return sp.status
+
+    def half():
+        s.solveEE(cuda.zeros_like(b), b, 0.3, S.SolverParams(r2req=1e-20, sloppySolve=S.L.SLOPPY_HALF))
+
+    with pytest.raises(S.L.QexStagError):
+        s.update_links(cuda.zeros_like(g))
+    for call in (shifted, half, lambda: s.bench_schur(1, 1), lambda: s.bench_schur(2, 1)):
+        with pytest.raises(S.L.QexStagError):
+            call()
+    s.update_links(g)
+    assert shifted() == S.L.OK
+    half()
