@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kSmBlock) link_update_kernel(int V, double2 *u
   m_load(x, p + off, (size_t)V, s);
   m_scale(x, eps);
   exp_ah(e, x);
-  m_load(y, u + off, (size_t)V, s);
+  m_load_own(y, u + off, (size_t)V, s);
   m_nn(z, e, y);
   m_store(u + off, (size_t)V, s, z);
 }

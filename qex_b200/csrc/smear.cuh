@@ -23,6 +23,12 @@ __device__ __forceinline__ void m_load(M3 &m, const double2 *f, size_t V, int s)
 #pragma unroll
   for (int e = 0; e < 9; e++) m.e[e] = __ldg(f + (size_t)e * V + s);
 }
+// a matrix of a field that this launch writes: not through the read-only path,
+// which is for data that stay as they are while a kernel runs
+__device__ __forceinline__ void m_load_own(M3 &m, const double2 *f, size_t V, int s) {
+#pragma unroll
+  for (int e = 0; e < 9; e++) m.e[e] = f[(size_t)e * V + s];
+}
 __device__ __forceinline__ void m_store(double2 *f, size_t V, int s, const M3 &m) {
 #pragma unroll
   for (int e = 0; e < 9; e++) f[(size_t)e * V + s] = m.e[e];

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kSmBlock, 2) fat7_adj_side_kernel(const AdjArg
   const double2 *Ud = A.u + d * A.ufs;
   M3 p;
   m_zero(p);
-  if (A.accumulate) m_load(p, A.d + d * A.dfs, V, c.site);
+  if (A.accumulate) m_load_own(p, A.d + d * A.dfs, V, c.site);
   const int syd = disp1(g, c.x, c.lex, c.par, d, 1);
 #pragma unroll 1
   for (int jm = 0; jm < 3; jm++) {
@@ -177,10 +177,7 @@ __global__ void __launch_bounds__(kSmBlock, 3) fat7_adj_link_kernel(const AdjArg
   const double2 *Ud = A.u + d * A.ufs;
   M3 acc;
   m_zero(acc);
-  if (A.accumulate || A.side) {
-#pragma unroll
-    for (int e = 0; e < 9; e++) acc.e[e] = A.d[d * A.dfs + (size_t)e * V + c.site];
-  }
+  if (A.accumulate || A.side) m_load_own(acc, A.d + d * A.dfs, V, c.site);
   {
     M3 md;
     m_load(md, A.m + d * A.mfs, V, c.site);
@@ -302,7 +299,7 @@ __global__ void __launch_bounds__(kSmBlock)
 #pragma unroll
     for (int e = 0; e < 9; e++) Y.e[e] = cmul(ad.e[e], idet);
   }
-  m_load(T, chain + off, (size_t)V, s);
+  m_load_own(T, chain + off, (size_t)V, s);  // out may be chain
   m_nn(R, T, Z);  // C Z
   m_load(T, u + off, (size_t)V, s);
   m_dn(Z, T, R);  // U^dag C Z
