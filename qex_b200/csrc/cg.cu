@@ -1,8 +1,8 @@
 // cg.cu -- FP64 conjugate gradient (src/solvers/cg.nim:55-272, precon
 // cpNone) on one parity of the Schur operator, with every scalar kept on the
-// device: the host only enqueues iterations and reads the CgState every few
-// iterations to see whether the solve is done.  Kernels launched after
-// convergence return at once (CgState.done), so the iteration count and the
+// device: the host keeps a few iterations queued ahead of the one that the
+// solve last reported (Pace) and reads the CgState at the end.  Kernels
+// launched after convergence return at once (CgState.done), so the iteration count and the
 // solution are those of QEX's loop
 //   while itn < maxits and r2 > r2stop:
 //     beta = rz/rzo; p = (itn == 0) ? r : r + beta p; itn++
@@ -203,12 +203,12 @@ int Pace::wait(unsigned long long *seen) {
   }
 }
 
-// iterations enqueued between host checks: small lattices run many
-// iterations per check (launch-bound), large ones few (each is long)
+// iterations that the solves on domains enqueue between host checks: small
+// lattices many (launch-bound), large ones few (each is long)
 int check_interval(int nh) {
   if (nh <= 1 << 14) return 64;
   if (nh <= 1 << 17) return 16;
-  return 8;  // 16 or 32 change a 32^4 16-bit solve by <= 1 %
+  return 8;
 }
 
 int cg64(qexstag_links_s *g, int par, double m2, CVecD b, VecD x, double r2req, int maxits,

@@ -23,7 +23,8 @@ namespace qs {
 
 struct DslashArgs64 {
   Geom g;
-  int po;
+  int po;  // output parity; with both in one launch (BOTH) unused: even blocks work
+           // on even sites, and the fields' pointers are those of the whole lattice
   const double2 *__restrict__ u;
   const double2 *__restrict__ xin;
   int istride;
@@ -44,9 +45,7 @@ struct DslashArgs64 {
   // instead nsites / rowlen runs of rowlen sites, pitch apart, from k0
   int k0, n1, k2, nsites;
   int rowlen, pitch;
-  // both parities in one launch (BOTH): even blocks on even sites; po is unused
-  // and the fields' pointers are those of the whole lattice
-  Progress progress;  // posted by this launch (a solve's first half sweep)
+  Progress progress;  // posted by this launch (one of an iteration's half sweeps)
   CgFused cg;         // fused CG (CG > 0)
 };
 
@@ -371,7 +370,9 @@ __global__ void __launch_bounds__(kBlock, CG ? 0 : 2) dslash64_split_kernel(cons
 //   23.8 / 27.0, 16^4 30.8 / 26.5 / 29.1, 16^3 x 24 43.0 / 42.9 / 36.6
 //   naive 14^4 10.4 / 11.3 / 12.9, 12^3 x 32 12.5 / 12.9 / 14.6, 16^4 15.5 / 14.5 /
 //   16.2, 16^3 x 24 21.9 / 25.1 / 20.9, 24^4 61.4 / 65.8 / 61.6
-//   D, fat+Naik 8^3 x 16 5.8 / 7.2 / 9.2, 12^4 9.5 / 8.4 / 10.4, 16^4 25.8 / 18.2 / 14.7
+//   D, fat+Naik 8^3 x 16 6.0 / 7.0 / 9.1, 8^3 x 32 7.2 / 7.7 / 9.9, 10^2 x 12 x 14 7.6 /
+//   7.9 / 10.2, 12^4 9.5 / 8.2 / 10.3, 16^4 25.5 / 18.0 / 14.5; naive the launch's 5.9
+//   in all three up to 10^2 x 12 x 14, 12^4 6.3 / 6.0 / 5.9, 16^4 16.3 / 10.6 / 8.4
 template <int NL, int BOTH>
 constexpr int kSplitMax = BOTH ? 16384 : NL == 8 ? 23000 : 30000;
 
@@ -556,10 +557,12 @@ int dslash64_rows(const qexstag_links_s *gl, int po, VecD out, CVecD xin, CVecD 
 
 // Whether an FP64 CG takes the fused iteration, whose sweeps are spread over
 // warps: on small lattices, and where the whole-site form would have a second
-// round of blocks (two on an SM) that is nearly empty.  Iteration us, fused /
-// not: fat+Naik 12^4 18 / 24.5, 12^3 x 32 32 / 36, 16^4 40.0 / 38.8, 16^3 x 32
-// 63 / 59, 20^4 (313 blocks for 296 places) 76 / 86, 24^4 151 / 147; naive 12^3 x 32
-// 21.5 / 27.3, 16^4 26.6 / 25.9, 16^3 x 32 41.5 / 38.5, 20^4 48 / 52, 24^4 87 / 85.
+// round of blocks (two on an SM) that is at most a third full.  Iteration us,
+// fused / not: fat+Naik 12^3 x 32 30 / 34, 16^4 38 / 37, 16^2 x 18 x 30 64 / 60; by
+// blocks for 296 places 297 72 / 80, 313 74 / 83, 325 75 / 84, 344 82 / 86, 366 87 / 89,
+// 375 88 / 90, 384 87 / 90, 395 95 / 92, 432 100 / 97; naive 12^3 x 32 19.2 / 24.8, 16^3 x
+// 14 21.5 / 25.6, 16^4 22.9 / 21.5, 270 blocks 40.9 / 38.0, 297 45.6 / 47.9, 325 47.2 /
+// 50.5, 344 51.8 / 51.4, 375 54.2 / 53.7, 384 53.7 / 53.7, 395 57.4 / 54.5.
 bool cg_fused_fits(const qexstag_links_s *gl) {
   const int nh = gl->l->g.nh, blocks = (nh + kBlock - 1) / kBlock, places = 2 * num_sms();
   return nh <= 30000 || (blocks > places && blocks <= places + places / 3);

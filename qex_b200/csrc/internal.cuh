@@ -255,9 +255,11 @@ struct CgState {
 
 // A running solve's report to the host, one 64-bit word in pinned memory:
 // iterations done, the flags below and the epoch (reliable updates done) they
-// belong to, from where the solve keeps them on the device.  The first half
-// sweep of an iteration posts it: a kernel is not over before such a write is
-// (about 2 us), and that kernel's own work covers the wait.
+// belong to, from where the solve keeps them on the device.  A half sweep of
+// each iteration posts it (the first one; the second in the fused CG, whose
+// first one sums |r|^2 before it knows whether the solve goes on): a kernel
+// is not over before such a write is (about 2 us), and its own work covers the
+// wait.
 struct Progress {
   unsigned long long *word = nullptr;
   const int *itn = nullptr, *stop = nullptr;

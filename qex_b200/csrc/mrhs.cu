@@ -241,11 +241,12 @@ __global__ void __launch_bounds__(kBlock, 3) dslashN64_ring_kernel(const DnArgs 
 }
 
 // The ring pays from about 260000 sites times vectors on; below, its barriers
-// cost more than its warps give.  us, first kernel / ring, fat+Naik: 16^4 (32768
-// sites a parity) 8 vectors 42 / 44; 20^4 3 vectors 50 / 52, 4 60 / 54, 8 102 /
-// 87; 24^4 3 vectors 95 / 89, 8 198 / 171; 32^4 3 vectors 411 / 300, 8 608 / 589;
-// naive 16^4 8 vectors 25 / 25, 20^4 3 29 / 30, 4 33 / 32, 32^4 8 353 / 304.  One
-// group, two vectors at most, has no use for it: 32^4 190 / 313.
+// cost more than its warps give, but for four vectors, which gain from 20^4 on.
+// us, first kernel / ring, fat+Naik: 16^4 (32768 sites a parity) 3 vectors 21.0 /
+// 24.9, 8 43.7 / 42.9; 20^4 3 51 / 52, 4 61 / 54, 8 103 / 85; 24^4 3 98 / 92, 4 118 /
+// 100, 8 212 / 171; 32^4 3 432 / 301, 4 372 / 313, 8 663 / 553; 24^3 x 48 8 422 / 336;
+// naive 16^4 8 25 / 25, 20^4 3 29 / 29, 4 34 / 31, 32^4 8 382 / 279.  One group, two
+// vectors at most, has no use for it: 32^4 190 / 313.
 constexpr long kDnRingFrom = 262144;
 
 template <int NL>

@@ -30,7 +30,7 @@ struct CgmState {
   int last;           // the iteration that ended the last live right-hand side
   int pad0;
   int live[kMaxRhs];  // right-hand side still iterating
-  double r2i[kMaxRhs], pAp[kMaxRhs], alpha[kMaxRhs], beta[kMaxRhs];
+  double r2i[kMaxRhs], pAp[kMaxRhs], beta[kMaxRhs];
   double alphaim1[kMaxRhs], betaim1[kMaxRhs], r2stop[kMaxRhs], b2[kMaxRhs];
   double sg[kMaxShift];
   double zi[kMaxRhs][kMaxShift], zim1[kMaxRhs][kMaxShift];

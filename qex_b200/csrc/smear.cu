@@ -17,7 +17,8 @@
 // and three sweeps: the 12 S fields, the 12 G fields (S read, G written
 // once), and fl: 9216 B and 48 staples per site where a field per staple
 // took 14976 B and 72.  At 32^4 the whole HISQ smear went from 13.03 to
-// 8.74 ms.  The unitary projection and the Naik product
+// 8.74 ms in runs of hundreds, which the power cap holds at 1.6 GHz, and from 11.8
+// to 7.7 ms in bursts at 1.965 GHz.  The unitary projection and the Naik product
 // naik U(x) U(x+mu) U(x+2mu) are one more sweep each.
 //
 // Fields are double2[4][9][V] (direction, element 3*row+col, site index of
