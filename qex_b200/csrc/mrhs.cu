@@ -240,21 +240,28 @@ __global__ void __launch_bounds__(kBlock, 3) dslashN64_ring_kernel(const DnArgs 
   }
 }
 
-// The ring pays from about 260000 sites times vectors on; below, its barriers
-// cost more than its warps give, but for four vectors, which gain from 20^4 on.
-// us, first kernel / ring, fat+Naik: 16^4 (32768 sites a parity) 3 vectors 21.0 /
-// 24.9, 8 43.7 / 42.9; 20^4 3 51 / 52, 4 61 / 54, 8 103 / 85; 24^4 3 98 / 92, 4 118 /
-// 100, 8 212 / 171; 32^4 3 432 / 301, 4 372 / 313, 8 663 / 553; 24^3 x 48 8 422 / 336;
-// naive 16^4 8 25 / 25, 20^4 3 29 / 29, 4 34 / 31, 32^4 8 382 / 279.  One group, two
-// vectors at most, has no use for it: 32^4 190 / 313.
-constexpr long kDnRingFrom = 262144;
+// The ring pays from about 260000 sites times vectors on for six and eight
+// vectors, and from 490000 on for any more than two; below, its barriers cost more
+// than its warps give.  In between an odd number leaves half of a group idle, and
+// with three or four a block's 128 sites make a last wave that is nearly empty on
+// some lattices (16^2 x 18 x 30: 540 blocks for 444 places).  us, first kernel / ring,
+// fat+Naik, by sites times vectors in thousands: 3 vectors 207 38 / 46, 288 53 / 60,
+// 498 97 / 89; 4 276 46 / 48, 327 62 / 56, 384 66 / 63, 664 112 / 97; 5 346 62 / 68, 480
+// 94 / 91, 829 196 / 161; 6 295 56 / 54, 415 75 / 70, 576 114 / 93; 7 344 50 / 56, 484 73 /
+// 72, 672 118 / 96; 8 262 43.7 / 42.9, 393 62 / 58, 553 83 / 75; naive 3 288 30 / 35, 498
+// 53 / 52; 4 276 27 / 29, 384 36.9 / 37.6, 664 64 / 56; 5 408 43 / 46, 829 101 / 79; 6 295
+// 31.7 / 31.6; 7 484 41.7 / 42.3, 672 68 / 55; 8 262 25 / 25, 393 35 / 34.  32^4 fat+Naik 3
+// vectors 432 / 301, 8 663 / 553; 24^3 x 48 8 422 / 336.  One group, two vectors at most,
+// has no use for it: 32^4 190 / 313.
+constexpr long kDnRingFromFull = 262144, kDnRingFrom = 490000;
 
 template <int NL>
 static void launch_dn(const DnArgs &A) {
   const long nh = A.g.nh;
   const int S = kBlock / A.groups;
   const int sets = (int)((nh + S - 1) / S);
-  if (A.groups == 1 || nh * A.n <= kDnRingFrom)
+  const long from = A.n == 6 || A.n == 8 ? kDnRingFromFull : kDnRingFrom;
+  if (A.groups == 1 || nh * A.n <= from)
     dslashN64_kernel<NL><<<std::min(sets, num_sms() * 4), kBlock, 0, stream()>>>(A);
   else if (A.groups == 2)
     dslashN64_ring_kernel<NL, 2><<<sets, kBlock, 0, stream()>>>(A);

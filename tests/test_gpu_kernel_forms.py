@@ -373,3 +373,11 @@ def test_no_reduced_precision_after_a_failed_update(cuda):
     s.update_links(g)
     assert shifted() == S.L.OK
     half()
+
+
+# the same from 490000 sites times vectors on, where the ring takes any number of
+# vectors above two: 171072 sites a parity are 1336 1/2 sets of 128 and 2673 of 64
+@pytest.mark.parametrize("n", [3, 4, 5, 7])
+@pytest.mark.parametrize("naik", [0, 1])
+def test_several_vectors_on_large_lattices(cuda, n, naik):
+    test_several_vectors_forms(cuda, (18, 22, 24, 36), n, naik)
