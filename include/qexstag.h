@@ -327,7 +327,9 @@ void qexstag_fat7_coefs_set_hisq(qexstag_fat7_coefs *c, double f7lf, double naik
 void qexstag_hisq_coefs_init(qexstag_hisq_coefs *c, double lepage, double naik);
 
 /* A smearing handle holds the device scratch of the staple sweeps (24 link
-   fields of 144 B per site, and 36 more for the chain rule, plus staging); it keeps a pointer to l. */
+   fields of 144 B per site, and 36 more for the chain rule, plus staging; for
+   a level of one-links alone none, with 3-staples too 12 for the chain rule);
+   it keeps a pointer to l. */
 typedef struct qexstag_smear_s qexstag_smear;
 int qexstag_smear_create(qexstag_layout *l, qexstag_smear **out);
 int qexstag_smear_destroy(qexstag_smear *s);

@@ -367,6 +367,8 @@ inline int smear_out_finish(qexstag_smear_s *s, const double2 *dev, double *p, i
 inline bool has_inner(const qexstag_fat7_coefs &c) {
   return c.five_staple != 0.0 || c.seven_staple != 0.0 || c.lepage != 0.0;
 }
+// a level whose links are side links of staples
+inline bool has_side(const qexstag_fat7_coefs &c) { return has_inner(c) || c.three_staple != 0.0; }
 inline int smear_scratch(qexstag_smear_s *s, const qexstag_fat7_coefs &c, double2 **s3, double2 **gm) {
   const Geom &g = s->l->g;
   const size_t f = sizeof(double2) * 9 * (size_t)g.V;

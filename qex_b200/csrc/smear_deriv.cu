@@ -351,7 +351,7 @@ int fat7_adj_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, s
   A.c3 = c.three_staple;
   A.c7 = c.seven_staple;
   A.inner = has_inner(c) ? 1 : 0;
-  A.side = (A.inner || A.c3 != 0.0) ? 1 : 0;
+  A.side = has_side(c) ? 1 : 0;
   A.q = q;
   int rc;
   if (A.inner && ((rc = staples_dev(g, u, ufs, m, mfs, t7)) ||
@@ -369,12 +369,13 @@ int fat7_adj_dev(const Geom &g, const qexstag_fat7_coefs &c, const double2 *u, s
 
 enum DerivSlot { kSdT7 = 40, kSdM3, kSdQ, kSdTmp, kSdDW, kSdIn2, kSdIn3 };
 
-static int adj_scratch(qexstag_smear_s *s, double2 **t7, double2 **m3, double2 **q) {
+// scratch of a level's adjoint (null where the level has no use for it)
+static int adj_scratch(qexstag_smear_s *s, const qexstag_fat7_coefs &lv, double2 **t7, double2 **m3, double2 **q) {
   const size_t f = sizeof(double2) * 9 * (size_t)s->l->g.V;
-  void *a, *b, *c;
+  void *a = nullptr, *b = nullptr, *c = nullptr;
   int rc;
-  if ((rc = s->ws.get(kSdT7, 12 * f, &a)) || (rc = s->ws.get(kSdM3, 12 * f, &b)) || (rc = s->ws.get(kSdQ, 12 * f, &c)))
-    return rc;
+  if (has_inner(lv) && ((rc = s->ws.get(kSdT7, 12 * f, &a)) || (rc = s->ws.get(kSdM3, 12 * f, &b)))) return rc;
+  if (has_side(lv) && (rc = s->ws.get(kSdQ, 12 * f, &c))) return rc;
   *t7 = (double2 *)a;
   *m3 = (double2 *)b;
   *q = (double2 *)c;
@@ -392,7 +393,7 @@ static int hisq_deriv_dev(qexstag_smear_s *s, const qexstag_hisq_coefs &c, const
   double2 *s3, *gm, *t7, *m3, *q;
   int rc;
   if ((rc = s->ws.get(kSmT1, field4_bytes(geo), &pv)) || (rc = s->ws.get(kSmW, field4_bytes(geo), &pw)) ||
-      (rc = s->ws.get(kSdDW, field4_bytes(geo), &pd)) || (rc = adj_scratch(s, &t7, &m3, &q)))
+      (rc = s->ws.get(kSdDW, field4_bytes(geo), &pd)))
     return rc;
   double2 *v = (double2 *)pv, *w = (double2 *)pw, *dw = (double2 *)pd;
   if (!forward) {
@@ -405,12 +406,13 @@ static int hisq_deriv_dev(qexstag_smear_s *s, const qexstag_hisq_coefs &c, const
     return rc;
   }
   // second level (fat7 and Naik both of w) -> dS/dw
-  if ((rc = fat7_adj_dev(geo, c.fat7second, w, fs, cf, cfs, cl, cls, c.naik, s3, gm, t7, m3, q, dw, fs, false)))
+  if ((rc = adj_scratch(s, c.fat7second, &t7, &m3, &q)) ||
+      (rc = fat7_adj_dev(geo, c.fat7second, w, fs, cf, cfs, cl, cls, c.naik, s3, gm, t7, m3, q, dw, fs, false)))
     return rc;
   // projectU -> dS/dv (in place)
   if ((rc = project_u_deriv_dev(geo, w, v, dw, dw, c.reunit_eps))) return rc;
   // first level: its inner fields again, then dS/dg
-  if ((rc = smear_scratch(s, c.fat7first, &s3, &gm))) return rc;
+  if ((rc = smear_scratch(s, c.fat7first, &s3, &gm)) || (rc = adj_scratch(s, c.fat7first, &t7, &m3, &q))) return rc;
   if (has_inner(c.fat7first) && (rc = fat7_inner_dev(geo, c.fat7first, g, fs, s3, gm))) return rc;
   return fat7_adj_dev(geo, c.fat7first, g, fs, dw, fs, nullptr, 0, 0.0, s3, gm, t7, m3, q, d, fs, false);
 }
@@ -477,7 +479,7 @@ int qexstag_fat7_deriv(qexstag_smear *s, const qexstag_fat7_coefs *c, const doub
       dl = (double2 *)dl0;
     }
   }
-  if ((rc = smear_scratch(s, *c, &s3, &gm)) || (rc = adj_scratch(s, &t7, &m3, &q))) return rc;
+  if ((rc = smear_scratch(s, *c, &s3, &gm)) || (rc = adj_scratch(s, *c, &t7, &m3, &q))) return rc;
   if (has_inner(*c) && (rc = fat7_inner_dev(geo, *c, u, fs, s3, gm))) return rc;
   if (same) {
     if ((rc = fat7_adj_dev(geo, *c, u, fs, m, fs, lmid, fs, naik, s3, gm, t7, m3, q, d, fs, true))) return rc;
@@ -490,8 +492,8 @@ int qexstag_fat7_deriv(qexstag_smear *s, const qexstag_fat7_coefs *c, const doub
       void *ptmp;
       if ((rc = s->ws.get(kSdTmp, field4_bytes(geo), &ptmp))) return rc;
       QS_CUDA(cudaMemsetAsync(ptmp, 0, field4_bytes(geo), stream()));
-      if ((rc = fat7_adj_dev(geo, z, ul, fs, (const double2 *)ptmp, fs, lmid, fs, naik, nullptr, nullptr, t7, m3, q, dl,
-                             fs, true)))
+      if ((rc = fat7_adj_dev(geo, z, ul, fs, (const double2 *)ptmp, fs, lmid, fs, naik, nullptr, nullptr, nullptr,
+                             nullptr, nullptr, dl, fs, true)))
         return rc;
     }
   }

@@ -381,3 +381,16 @@ def test_no_reduced_precision_after_a_failed_update(cuda):
 @pytest.mark.parametrize("naik", [0, 1])
 def test_several_vectors_on_large_lattices(cuda, n, naik):
     test_several_vectors_forms(cuda, (18, 22, 24, 36), n, naik)
+
+
+# a chain rule without terms beyond the 3-staple takes no scratch for them: at
+# most the 28 link fields that it has always held
+@pytest.mark.parametrize("coef", [[0.5, 0.0, 0.0, 0.0, 0.0], [0.4, 0.2, 0.0, 0.0, 0.0]])
+def test_chain_rule_scratch_of_simple_levels(cuda, coef):
+    dims = (16, 16, 16, 16)
+    u = cuda.zeros((4, 3, 3, F.volume(dims)), dtype=cuda.complex128, device="cuda")
+    d, sm = cuda.zeros_like(u), SM.Smear(S.Layout(dims))
+    cuda.cuda.synchronize()
+    free = cuda.cuda.mem_get_info()[0]
+    sm.fat7Deriv(d, u, u, SM.Fat7lCoefs(*coef))
+    assert free - cuda.cuda.mem_get_info()[0] <= 28 * 144 * F.volume(dims) + (8 << 20)
