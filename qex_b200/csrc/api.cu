@@ -119,6 +119,14 @@ int Workspace::get(int slot, size_t bytes, void **out) {
   return QEXSTAG_OK;
 }
 
+void Workspace::drop(int slot) {
+  auto it = bufs.find(slot);
+  if (it == bufs.end()) return;
+  cudaStreamSynchronize(stream());
+  cudaFree(it->second.second);
+  bufs.erase(it);
+}
+
 int Workspace::get_pinned(size_t bytes, void **out) {
   if (pinned && pinned_bytes >= bytes) {
     *out = pinned;

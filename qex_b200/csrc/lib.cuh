@@ -20,6 +20,7 @@ struct Workspace {
   size_t pinned_bytes = 0;
   unsigned long long *progress = nullptr;  // pinned word a running solve reports through
   int get(int slot, size_t bytes, void **out);
+  void drop(int slot);  // frees a slot's buffer
   int get_pinned(size_t bytes, void **out);
   int get_progress(unsigned long long **out);
   void release();

@@ -860,8 +860,10 @@ static int shifted_residual(qexstag_links_s *g, double m2s, const double2 *bfull
   return vnorm2(CVecD{r, nh}, nh, r2);
 }
 
-int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nrhs, const double2 *const *b,
-           double2 *const *y, const qexstag_solver_params *p, qexstag_solver_stats *st, double *r2_out) {
+// even: no odd number of right-hand sides above one at a time
+static int cgm_ee_run(qexstag_links_s *g, double m, int nshift, const double *sigma, int nrhs, const double2 *const *b,
+                      double2 *const *y, const qexstag_solver_params *p, qexstag_solver_stats *st, double *r2_out,
+                      bool even) {
   const Geom &geo = g->l->g;
   const int V = geo.V, nh = geo.nh;
   if (nshift > kMaxShift) return fail(QEXSTAG_ERR_ARG, "cgm_ee: at most 32 shifts");
@@ -886,8 +888,9 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
     if ((rc = vzero(block(y[i], geo, 1), nh))) return rc;
   // multi-shift phase, in batches of up to 8 right-hand sides
   const double r2ms = sloppy ? std::max(p->r2req, 1e-12) : p->r2req;
-  for (int j0 = 0; j0 < nrhs; j0 += kMaxRhs) {
-    const int nr = std::min(kMaxRhs, nrhs - j0);
+  for (int j0 = 0, nr; j0 < nrhs; j0 += nr) {
+    nr = std::min(kMaxRhs, nrhs - j0);
+    if (even && nr > 1) nr &= ~1;
     const double2 *bb[kMaxRhs];
     double2 *yy[kMaxRhs * kMaxShift];
     for (int j = 0; j < nr; j++) {
@@ -946,7 +949,7 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
         std::vector<double> r2(nr);
         for (int j = 0; j < nr; j++)
           if ((rc = shifted_residual(g, m2s, b[j0 + j], y[(j0 + j) * nshift + k], rbuf[j], t, &r2[j]))) return rc;
-        for (int pass = 0; pass < 10 && st->iterations < maxits; pass++) {
+        for (int pass = 0; pass < (even ? 20 : 10) && st->iterations < maxits; pass++) {
           // systems still above target, packed to the front
           std::vector<int> live;
           double req = 1.0;
@@ -958,6 +961,7 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
             }
           }
           if (live.empty()) break;
+          if (even && live.size() > 1 && live.size() % 2) live.pop_back();  // its turn comes in another pass
           req = std::max(req, 1e-12);  // what an FP32 inner solve can reach
           const double2 *rb[kMaxRhs];
           double2 *dy[kMaxRhs];
@@ -1031,6 +1035,18 @@ int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nr
   }
   st->r2 = worst;
   return status;
+}
+
+int cgm_ee(qexstag_links_s *g, double m, int nshift, const double *sigma, int nrhs, const double2 *const *b,
+           double2 *const *y, const qexstag_solver_params *p, qexstag_solver_stats *st, double *r2_out) {
+  const qexstag_solver_stats start = *st;
+  const int rc = cgm_ee_run(g, m, nshift, sigma, nrhs, b, y, p, st, r2_out, false);
+  if (rc != QEXSTAG_ERR_ALLOC || p->sloppy == QEXSTAG_SLOPPY_NONE || nrhs % kMaxRhs == 1 || nrhs % 2 == 0) return rc;
+  // memory is short, and the pair of an odd right-hand side is half empty:
+  // once more with the odd one by itself
+  for (int k = 40; k <= 44; k++) g->ws.drop(kSlotMs0 + k);
+  *st = start;
+  return cgm_ee_run(g, m, nshift, sigma, nrhs, b, y, p, st, r2_out, true);
 }
 
 }  // namespace qs
